@@ -56,6 +56,8 @@ struct AttnDecodeArgs {
     int keep, fixed_tokens;
     // one value per query head whose exponential joins the softmax's denominator; null: none
     const float* sink;
+    // > 0: the blocks are shared out by the rows' own lengths (share_out): blocks per kv head
+    int slots;
 };
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
@@ -148,6 +150,79 @@ __device__ __forceinline__ void join_runs_by_warp(const float* unit_partial, int
     }
 }
 
+// How many tiles of 16 keys a row at position `pos` walks: the kept first positions' (up to
+// `kept_tiles`) and the window's or chunk's or everything's, from tile `tile_lo` on.
+__device__ __forceinline__ int tiles_of(const AttnDecodeArgs& p, int pos, int* kept_tiles, int* tile_lo) {
+    const int lo = first_visible(pos, p.window, p.chunk);
+    *kept_tiles = (kept_before(lo, p.keep) + 15) >> 4;
+    *tile_lo = max(lo >> 4, *kept_tiles);
+    return *kept_tiles + max(0, (pos >> 4) - *tile_lo + 1);
+}
+
+// The most rows whose blocks are shared out by their lengths (a lane keeps MAX_SHARED / 32 of them).
+constexpr int MAX_SHARED_ROWS = 128;
+
+// A step's sequences are seldom equally long, and a launch that cuts every row into the same
+// number of runs lasts as long as the longest row's: 64 sequences of 150 to 3 001 positions (4 kv
+// heads of 256) took 98 us where their keys and values take 38 at the copy bandwidth.  So every
+// block finds its place itself: with `each` tiles a warp, row r gets ceil(tiles_r / (nw each))
+// blocks per kv head, and `each` is the smallest number at which that fits the `slots` blocks
+// there are (all resident at once) and no row needs more than MAX_SPLITS.  It depends on the rows'
+// positions alone, which the host wrote before the step, so it runs ahead of pdl_wait; every warp
+// does it for itself, without a barrier.  Returns false for a block that is left over.
+__device__ __forceinline__ bool share_out(const AttnDecodeArgs& p, int slot, int nw, int lane, int* row,
+                                          int* split, int* splits, int* first_slot) {
+    constexpr int PER_LANE = MAX_SHARED_ROWS / 32;
+    int tiles[PER_LANE], total = 0, most = 0;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int r = lane + 32 * i;
+        int kept_tiles, tile_lo;
+        tiles[i] = r < p.rows ? tiles_of(p, p.row_pos[r], &kept_tiles, &tile_lo) : 0;
+        total += tiles[i];
+        most = max(most, tiles[i]);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    most = __reduce_max_sync(0xffffffffu, most);
+    // Bounds of `each`: the blocks' warps take all tiles at least; a row wastes less than a block.
+    int lo = max((total + p.slots * nw - 1) / (p.slots * nw), (most + MAX_SPLITS * nw - 1) / (MAX_SPLITS * nw));
+    int hi = (most + nw - 1) / nw;                 // one block a row
+    if (p.slots > p.rows) hi = min(hi, (total + (p.slots - p.rows) * nw - 1) / ((p.slots - p.rows) * nw));
+    lo = max(lo, 1);
+    hi = max(hi, lo);
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1, q = mid * nw;
+        int need = 0;
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i) need += (tiles[i] + q - 1) / q;
+        if ((int)__reduce_add_sync(0xffffffffu, need) <= p.slots) hi = mid;
+        else lo = mid + 1;
+    }
+    const int q = lo * nw;
+    int before = 0;                                // blocks of the rows of earlier rounds
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int mine = (tiles[i] + q - 1) / q;
+        int upto = mine;                           // blocks up to and with this lane's row
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned found = __ballot_sync(0xffffffffu, slot < before + upto);
+        if (found) {
+            const int at = __ffs(found) - 1;
+            *row = at + 32 * i;
+            *splits = __shfl_sync(0xffffffffu, mine, at);
+            *first_slot = before + __shfl_sync(0xffffffffu, upto, at) - *splits;
+            *split = slot - *first_slot;
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
 // HD: head size (64, 128 or 256).  G: query heads per kv head (1, 2, 4 or 8).  EARLY: the first
 // tile of keys may be fetched before the kernel ahead of this one has finished (it shortens
 // the chain of waits of a step of one row: batch 1 runs 1.5 % faster with it; with more rows
@@ -155,7 +230,9 @@ __device__ __forceinline__ void join_runs_by_warp(const float* unit_partial, int
 // and batch 8 2 % slower with it).
 // WIDE: blocks of 8 warps (a single row's step: half as many partial results to join as with
 // blocks of 4); the narrower kernel keeps its registers and shared memory as they were.
-template <int HD, int G, bool EARLY, bool WIDE = false>
+// SHARED: the blocks of a kv head are shared out by the rows' lengths (share_out), else every row
+// has `splits` of them.
+template <int HD, int G, bool EARLY, bool WIDE = false, bool SHARED = false>
 __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(AttnDecodeArgs p) {
     constexpr int KB = HD / 32;          // 32-wide blocks of the head dimension
     constexpr int LPK = HD / 8;          // lanes that cover one value row
@@ -172,9 +249,15 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     float(*s_sm)[8] = sm_all[warp][0];
     float(*p_sm)[8] = sm_all[warp][1];
     pdl_trigger();
-    const int split = (int)(blockIdx.x % p.splits);
-    const int kvh = (int)((blockIdx.x / p.splits) % p.n_kv);
-    const int r = (int)(blockIdx.x / ((unsigned)p.splits * p.n_kv));
+    int split, kvh, r, splits = p.splits, first_slot = 0;
+    if (SHARED) {
+        kvh = (int)(blockIdx.x % p.n_kv);
+        if (!share_out(p, (int)(blockIdx.x / p.n_kv), nw, lane, &r, &split, &splits, &first_slot)) return;
+    } else {
+        split = (int)(blockIdx.x % splits);
+        kvh = (int)((blockIdx.x / splits) % p.n_kv);
+        r = (int)(blockIdx.x / ((unsigned)splits * p.n_kv));
+    }
     const int g = lane >> 2, t = lane & 3;
 
     // Where the row is and which pages it reads: written by the host before the step, not
@@ -186,11 +269,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     // not one of those; a tile's number `v` in that order is position tile v, or v + skip from
     // the window on.
     const int n_kept = kept_before(lo, p.keep);
-    const int kept_tiles = (n_kept + 15) >> 4;
-    const int tile_lo = max(lo >> 4, kept_tiles), tile_hi = pos >> 4;             // inclusive
+    int kept_tiles, tile_lo;
+    const int n_tiles = tiles_of(p, pos, &kept_tiles, &tile_lo);
     const int skip = tile_lo - kept_tiles;
-    const int n_tiles = kept_tiles + max(0, tile_hi - tile_lo + 1);
-    const int per = (n_tiles + nw * p.splits - 1) / (nw * p.splits);
+    const int per = (n_tiles + nw * splits - 1) / (nw * splits);
     const int t0 = (split * nw + warp) * per;
     const int t1 = min(t0 + per, n_tiles);
     auto tile_at = [&](int v) { return v < kept_tiles ? v : v + skip; };
@@ -325,7 +407,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     }
     __syncthreads();
     __nv_bfloat16* out_row = p.out + (size_t)r * p.n_heads * HD + (size_t)kvh * G * HD;
-    float* my_partial = p.partial + (((size_t)r * p.n_heads + kvh * G) * p.splits + split) * PW;
+    // the (row, kv head)'s partial results: [G][splits][PW]
+    float* unit_partial = p.partial + (SHARED ? ((size_t)kvh * p.slots + first_slot) * G * PW
+                                              : ((size_t)r * p.n_heads + kvh * G) * splits * PW);
+    float* my_partial = unit_partial + (size_t)split * PW;
     // (every thread makes the warps' weights for its head itself: no thread's loop and no
     // second barrier between the warps' results and their sum)
     for (int item = threadIdx.x; item < G * HD / 2; item += blockDim.x) {
@@ -342,27 +427,26 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
             a.x += f * v.x;
             a.y += f * v.y;
         }
-        if (p.splits == 1) {
+        if (splits == 1) {
             if (p.sink) sum += expf(p.sink[kvh * G + h] - mx);
             const float inv = 1.0f / sum;
             *reinterpret_cast<__nv_bfloat162*>(out_row + h * HD + d) =
                 __floats2bfloat162_rn(a.x * inv, a.y * inv);
         } else {
-            float* pp = my_partial + (size_t)h * p.splits * PW;
+            float* pp = my_partial + (size_t)h * splits * PW;
             if (d == 0) *reinterpret_cast<float2*>(pp) = make_float2(mx, sum);
             *reinterpret_cast<float2*>(pp + 2 + d) = a;
         }
     }
-    if (p.splits == 1) return;
+    if (splits == 1) return;
 
     // ---- the block that finishes last joins the splits ----
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) ticket_sm = atomicAdd(p.tickets + r * p.n_kv + kvh, 1);
     __syncthreads();
-    if (ticket_sm != p.splits - 1) return;
+    if (ticket_sm != splits - 1) return;
     __threadfence();
-    const float* unit_partial = p.partial + ((size_t)r * p.n_heads + kvh * G) * p.splits * PW;
     const float* sink_g = p.sink ? p.sink + kvh * G : nullptr;
     // Few enough runs and columns for a warp to join its columns by itself (before: maxima, a
     // barrier, one thread's loop over the runs, a barrier, the sums' loads, a barrier, a loop,
@@ -370,21 +454,21 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     {
         constexpr int ITEMS = G * HD / 2;
         bool joined = true;
-        if (WIDE && ITEMS <= 256 && p.splits <= 32)
-            join_runs_by_warp<HD, G, 1, 32>(unit_partial, p.splits, out_row, lane, sink_g);
-        else if (WIDE && ITEMS <= 256 && p.splits <= 64)
-            join_runs_by_warp<HD, G, 1, 64>(unit_partial, p.splits, out_row, lane, sink_g);
-        else if (WIDE && ITEMS <= 512 && p.splits <= 32)
-            join_runs_by_warp<HD, G, 2, 32>(unit_partial, p.splits, out_row, lane, sink_g);
-        else if (!WIDE && ITEMS <= (int)blockDim.x && p.splits <= 32)
-            join_runs_by_warp<HD, G, 1, 32>(unit_partial, p.splits, out_row, lane, sink_g);
-        else if (!WIDE && ITEMS <= 2 * (int)blockDim.x && p.splits <= 16)
-            join_runs_by_warp<HD, G, 2, 16>(unit_partial, p.splits, out_row, lane, sink_g);
-        else if (!WIDE && HD == 256 && ITEMS <= 2 * (int)blockDim.x && p.splits <= 32) {
+        if (WIDE && ITEMS <= 256 && splits <= 32)
+            join_runs_by_warp<HD, G, 1, 32>(unit_partial, splits, out_row, lane, sink_g);
+        else if (WIDE && ITEMS <= 256 && splits <= 64)
+            join_runs_by_warp<HD, G, 1, 64>(unit_partial, splits, out_row, lane, sink_g);
+        else if (WIDE && ITEMS <= 512 && splits <= 32)
+            join_runs_by_warp<HD, G, 2, 32>(unit_partial, splits, out_row, lane, sink_g);
+        else if (!WIDE && ITEMS <= (int)blockDim.x && splits <= 32)
+            join_runs_by_warp<HD, G, 1, 32>(unit_partial, splits, out_row, lane, sink_g);
+        else if (!WIDE && ITEMS <= 2 * (int)blockDim.x && splits <= 16)
+            join_runs_by_warp<HD, G, 2, 16>(unit_partial, splits, out_row, lane, sink_g);
+        else if (!WIDE && HD == 256 && ITEMS <= 2 * (int)blockDim.x && splits <= 32) {
             // (only where the loop over the keys needs as many registers anyway: at smaller
             // head sizes this would cost a resident block)
             if constexpr (HD == 256)
-                join_runs_by_warp<HD, G, 2, 32>(unit_partial, p.splits, out_row, lane, sink_g);
+                join_runs_by_warp<HD, G, 2, 32>(unit_partial, splits, out_row, lane, sink_g);
         }
         else
             joined = false;
@@ -393,18 +477,18 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
             return;
         }
     }
-    for (int i = threadIdx.x; i < G * p.splits; i += blockDim.x)
-        w_sm[i / p.splits][i % p.splits] = __ldcg(unit_partial + (size_t)i * PW);       // the maxima
+    for (int i = threadIdx.x; i < G * splits; i += blockDim.x)
+        w_sm[i / splits][i % splits] = __ldcg(unit_partial + (size_t)i * PW);       // the maxima
     __syncthreads();
     if (threadIdx.x < G) {
         const int h = threadIdx.x;
         float mx = -INFINITY;
-        for (int b = 0; b < p.splits; ++b) mx = fmaxf(mx, w_sm[h][b]);
+        for (int b = 0; b < splits; ++b) mx = fmaxf(mx, w_sm[h][b]);
         ml_sm[h][0] = mx;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < G * p.splits; i += blockDim.x) {
-        const int h = i / p.splits, b = i % p.splits;
+    for (int i = threadIdx.x; i < G * splits; i += blockDim.x) {
+        const int h = i / splits, b = i % splits;
         const float mb = w_sm[h][b];
         const float f = mb == -INFINITY ? 0.f : expf(mb - ml_sm[h][0]);
         w_sm[h][b] = f;
@@ -414,7 +498,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     if (threadIdx.x < G) {
         const int h = threadIdx.x;
         float sum = 0.f;
-        for (int b = 0; b < p.splits; ++b) sum += l_sm[h][b];        // in run order
+        for (int b = 0; b < splits; ++b) sum += l_sm[h][b];        // in run order
         if (sink_g) sum += expf(sink_g[h] - ml_sm[h][0]);
         ml_sm[h][1] = sum;
     }
@@ -422,10 +506,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
     // the weighted sum of the runs' accumulators, 8 loads in flight per thread
     for (int item = threadIdx.x; item < G * HD / 2; item += blockDim.x) {
         const int h = item / (HD / 2), d = 2 * (item % (HD / 2));
-        const float* pp = unit_partial + (size_t)h * p.splits * PW + 2 + d;
+        const float* pp = unit_partial + (size_t)h * splits * PW + 2 + d;
         float2 a = make_float2(0.f, 0.f);
         int b = 0;
-        for (; b + 8 <= p.splits; b += 8) {
+        for (; b + 8 <= splits; b += 8) {
             float2 v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
@@ -437,7 +521,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(Attn
                 a.y += f * v[u].y;
             }
         }
-        for (; b < p.splits; ++b) {
+        for (; b < splits; ++b) {
             const float f = w_sm[h][b];
             const float2 v = __ldcg(reinterpret_cast<const float2*>(pp + (size_t)b * PW));
             a.x += f * v.x;
@@ -516,7 +600,8 @@ static int attention_decode(
     int max_pages, int page_tokens, int ring_tokens, const int* row_pos, const int* row_seq,
     const int* seq_slot, void* out, float* partial, int* tickets, int rows, int n_heads, int n_kv,
     int head_dim, float scale, float softcap, int window, int splits, int warps, int fresh,
-    void* stream, int chunk = 0, const float* sink = nullptr, int keep = 0, int fixed_tokens = 0) {
+    void* stream, int chunk = 0, const float* sink = nullptr, int keep = 0, int fixed_tokens = 0,
+    int slots = 0) {
     if (rows == 0) return 0;
     SIB_REQUIRE(chunk >= 0 && (chunk == 0 || window == 0), "attention_decode: chunk=%d window=%d (a chunk "
                 "goes without a window)", chunk, window);
@@ -532,8 +617,11 @@ static int attention_decode(
                 "attention_decode: rows=%d splits=%d (1 to %d)", rows, splits, MAX_SPLITS);
     SIB_REQUIRE(warps == 1 || warps == 2 || warps == 4 || warps == 8,
                 "attention_decode: %d warps a block; 1, 2, 4 or 8", warps);
-    SIB_REQUIRE(splits == 1 || (partial != nullptr && tickets != nullptr &&
-                                ((uintptr_t)partial % 16) == 0),
+    SIB_REQUIRE(slots == 0 || (slots >= rows && rows <= MAX_SHARED_ROWS && warps <= 4),
+                "attention_decode: %d blocks a kv head for %d rows (at least one each, %d rows at most, blocks "
+                "of up to 4 warps)", slots, rows, MAX_SHARED_ROWS);
+    SIB_REQUIRE((splits == 1 && slots == 0) || (partial != nullptr && tickets != nullptr &&
+                                                ((uintptr_t)partial % 16) == 0),
                 "attention_decode: %d splits need memory for their partial results and the "
                 "ticket counters of the (row, kv head) pairs", splits);
     SIB_REQUIRE(k_pool && v_pool && page_table && max_pages > 0,
@@ -546,8 +634,8 @@ static int attention_decode(
     AttnDecodeArgs p{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
                      (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, partial, tickets, row_pos, row_seq,
                      seq_slot, page_table, q_stride, rows, n_heads, n_kv, max_pages, page_tokens,
-                     ring_tokens, window, splits, scale, softcap, fresh, chunk, keep, fixed_tokens, sink};
-    const long long blocks = (long long)rows * n_kv * splits;
+                     ring_tokens, window, splits, scale, softcap, fresh, chunk, keep, fixed_tokens, sink, slots};
+    const long long blocks = slots ? (long long)slots * n_kv : (long long)rows * n_kv * splits;
     SIB_REQUIRE(blocks < (1ll << 31), "attention_decode: too many rows (%d)", rows);
     cudaStream_t s = (cudaStream_t)stream;
     const int G = n_heads / n_kv;
@@ -563,7 +651,11 @@ static int attention_decode(
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                      \
                                  (int)((size_t)warps * GG * (HD + 2) * sizeof(float)));            \
         }                                                                                          \
-        if (warps == 8 && early_keys)                                                              \
+        if (slots)                                                                                 \
+            sib_launch_chained(attention_decode_kernel<HD, GG, false, false, true>,                \
+                               dim3((unsigned)blocks), dim3(32 * warps),                           \
+                               (size_t)warps * GG * (HD + 2) * sizeof(float), s, p);               \
+        else if (warps == 8 && early_keys)                                                         \
             sib_launch_chained(attention_decode_kernel<HD, GG, true, true>, dim3((unsigned)blocks), \
                                dim3(32 * warps), (size_t)warps * GG * (HD + 2) * sizeof(float), s, p); \
         else if (warps == 8)                                                                       \
@@ -631,6 +723,24 @@ SIB_EXPORT int sib_attention_decode_masked(
                             n_heads, n_kv, head_dim, scale, softcap, window, splits, warps, fresh,
                             stream, chunk, sink, keep, fixed_tokens);
 }
+
+// The same with the blocks shared out by the rows' lengths: `slots` blocks of `warps` warps per kv
+// head (at least one a row; all of them should be resident at once), up to MAX_SHARED_ROWS rows.
+// `partial`: [n_kv, slots, n_heads / n_kv, head_dim + 2].
+SIB_EXPORT int sib_attention_decode_shared_out(
+    const void* q, int q_stride, const void* k_pool, const void* v_pool, const int* page_table,
+    int max_pages, int page_tokens, int ring_tokens, const int* row_pos, const int* row_seq,
+    const int* seq_slot, void* out, float* partial, int* tickets, int rows, int n_heads, int n_kv,
+    int head_dim, float scale, float softcap, int window, int slots, int warps, int chunk,
+    const float* sink, int keep, int fixed_tokens, void* stream) {
+    SIB_REQUIRE(slots > 0, "attention_decode: %d blocks a kv head", slots);
+    return attention_decode(q, q_stride, k_pool, v_pool, page_table, max_pages, page_tokens,
+                            ring_tokens, row_pos, row_seq, seq_slot, out, partial, tickets, rows,
+                            n_heads, n_kv, head_dim, scale, softcap, window, 1, warps, 0, stream,
+                            chunk, sink, keep, fixed_tokens, slots);
+}
+
+SIB_EXPORT int sib_attention_decode_max_shared_rows() { return MAX_SHARED_ROWS; }
 
 // ---------------------------------------------------------------------------
 // The same kernels for callers that cannot allocate (attention_decode_no_alloc.h):

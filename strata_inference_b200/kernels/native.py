@@ -1582,7 +1582,7 @@ def attention_decode_resident_warps(n_heads: int, n_kv: int, head_dim: int, warp
 
 @_timed(lambda q, q_stride, k_pool, v_pool, page_table, page_tokens, ring_tokens, row_pos, row_seq,
         seq_slot, out, scratch, tickets, n_heads, n_kv, head_dim, scale, softcap, window, splits,
-        warps=4, fresh=0, chunk=0, sink=None, keep=0, fixed_tokens=0: _attention_cache_work(
+        warps=4, fresh=0, chunk=0, sink=None, keep=0, fixed_tokens=0, slots=0: _attention_cache_work(
             "attention_decode", row_pos, k_pool, n_heads, head_dim, window, out.shape[0], chunk=chunk,
             keep=keep))
 def attention_decode(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor, v_pool: torch.Tensor,
@@ -1592,7 +1592,7 @@ def attention_decode(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor, v_poo
                      scale: float, softcap: float, window: int, splits: int,
                      warps: int = 4, fresh: int = 0, chunk: int = 0,
                      sink: Optional[torch.Tensor] = None, keep: int = 0,
-                     fixed_tokens: int = 0) -> torch.Tensor:
+                     fixed_tokens: int = 0, slots: int = 0) -> torch.Tensor:
     """Attention of single rows over the bfloat16 cache (see csrc/attention_decode.cu).
     ``splits`` blocks of ``warps`` warps share the keys of a (row, kv head); with more than one they
     need ``scratch`` for their partial results and ``tickets``: int32 counters, one
@@ -1602,7 +1602,9 @@ def attention_decode(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor, v_poo
     runs.  0: every load waits for it.  ``chunk`` > 0 (without a window): a row sees the
     positions of its own chunk; ``sink``: one 32-bit value per query head whose exponential
     joins the softmax's denominator; ``keep`` > 0 (with a window): the sequence's first ``keep``
-    positions stay visible, ``fixed_tokens`` positions lie ahead of the ring."""
+    positions stay visible, ``fixed_tokens`` positions lie ahead of the ring.  ``slots`` > 0: that
+    many blocks per kv head are shared out among the rows by their lengths (``splits`` and
+    ``fresh`` do not count then); they take ``scratch`` for ``slots`` runs of one row."""
     global _launches
     rows = out.shape[0]
     _want(out, torch.bfloat16, "out")
@@ -1613,14 +1615,24 @@ def attention_decode(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor, v_poo
         raise KernelError("attention_decode: q must be bfloat16")
     if tuple(k_pool.shape[1:]) != (n_kv, page_tokens, head_dim):
         raise KernelError("attention_decode: pool layout must be [pages, kv_heads, page_tokens, head_dim]")
-    if splits > 1:
-        need = attention_rows_scratch_bytes(rows, n_heads, head_dim, splits)
+    if splits > 1 or slots:
+        need = attention_rows_scratch_bytes(1, n_heads, head_dim, slots) if slots else \
+            attention_rows_scratch_bytes(rows, n_heads, head_dim, splits)
         if scratch is None or scratch.numel() * scratch.element_size() < need:
             raise KernelError(f"attention_decode: {need} bytes of scratch memory are needed")
         if tickets is None or tickets.dtype != torch.int32 or tickets.numel() < rows * n_kv:
             raise KernelError(f"attention_decode: {rows * n_kv} int32 ticket counters are needed")
     if sink is not None:
         _f32(sink, n_heads, "sink")
+    if slots:
+        _check(library().sib_attention_decode_shared_out(
+            _ptr(q), c_int(q_stride), _ptr(k_pool), _ptr(v_pool), _ptr(page_table),
+            c_int(page_table.shape[1]), c_int(page_tokens), c_int(ring_tokens), _ptr(row_pos),
+            _ptr(row_seq), _ptr(seq_slot), _ptr(out), _ptr(scratch), _ptr(tickets), c_int(rows),
+            c_int(n_heads), c_int(n_kv), c_int(head_dim), c_float(scale), c_float(softcap),
+            c_int(window), c_int(slots), c_int(warps), c_int(chunk), _ptr(sink), c_int(keep),
+            c_int(fixed_tokens), _stream()))
+        return out
     _check(library().sib_attention_decode_masked(
         _ptr(q), c_int(q_stride), _ptr(k_pool), _ptr(v_pool), _ptr(page_table),
         c_int(page_table.shape[1]), c_int(page_tokens), c_int(ring_tokens), _ptr(row_pos),
@@ -1629,6 +1641,11 @@ def attention_decode(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor, v_poo
         c_int(window), c_int(splits), c_int(warps), c_int(fresh), c_int(chunk), _ptr(sink),
         c_int(keep), c_int(fixed_tokens), _stream()))
     return out
+
+
+def attention_decode_max_shared_rows() -> int:
+    """The most rows whose blocks ``attention_decode`` shares out by their lengths."""
+    return int(library().sib_attention_decode_max_shared_rows())
 
 
 def attention_prefill_supports(n_heads: int, n_kv: int, head_dim: int) -> bool:

@@ -156,6 +156,26 @@ def decode_shape(units: int, longest: int, window: int, resident4: int, resident
     return trimmed(min(most, 128), 1)
 
 
+def shared_shape(rows: int, n_kv: int, tiles: int, resident: int):
+    """(blocks per kv head, warps a block) of the decode kernel for ``rows`` rows of up to ``tiles``
+    tiles of 16 keys that share the blocks out by their lengths, on a device that holds
+    ``resident`` warps of the kernel; None where not even blocks of one warp go round.  Wide blocks
+    leave fewer partial results to join, narrow ones divide the keys more evenly: a narrower one is
+    taken where a warp of equally long rows would walk a fifth fewer tiles (64 rows of 3 000
+    positions, 4 kv heads of 256: 128 us with 2 warps, 140 with 4; 16 rows of 1 000: 21 with 2, 17 with
+    4), or where the wider blocks are hardly more than the rows and lengths could not count (100
+    rows of 64 to 7 000 positions, 8 kv heads of 256: 188 us with 1 warp, 297 with 2)."""
+    best, best_each = None, 0
+    for warps in (4, 2, 1):
+        slots = resident // (warps * n_kv)
+        if slots < rows or (warps > 1 and slots < 1.5 * rows):
+            continue
+        each = -(-tiles // (slots // rows * warps))
+        if best is None or each <= 0.8 * best_each:
+            best, best_each = (slots, warps), each
+    return best
+
+
 class Attention:
     chain_safe = True      # deferred results are read by this runtime's and native's launchers only
 
@@ -395,6 +415,26 @@ class Attention:
         want = max(1, self._target_warps // max(1, ctx.n_rows * self.nh))
         return max(1, min(want, -(-self._longest(ctx, capacity) // 32), 128))
 
+    def _decode_launch(self, ctx):
+        """(runs, warps, slots, scratch, tickets) of the decode kernel: blocks shared out by the
+        rows' lengths where ``shared_shape`` has a shape for it, else as many for every row."""
+        rt, R = self.rt, ctx.n_rows
+        runs, warps = self._decode_shape(ctx, ctx.cache.max_seq_len)
+        # (few (row, kv head) pairs have many runs each, and joining those costs more than unequal
+        # lengths do: 5 rows of 100 to 5 000 positions and one kv head take 12 us with blocks of 8
+        # warps, 27 shared out)
+        if warps < 8 and 1 < R <= native.attention_decode_max_shared_rows():
+            shared = shared_shape(R, self.nkv, -(-self._longest(ctx, ctx.cache.max_seq_len) // 16),
+                                  self._resident_warps[4])
+            if shared is not None:
+                slots, warps = shared
+                scratch = rt.scratch(native.attention_rows_scratch_bytes(1, self.nh, self.kw, slots))
+                return 1, warps, slots, scratch, rt.tickets(R * self.nkv)
+        if runs == 1:
+            return runs, warps, 0, None, None
+        scratch = rt.scratch(native.attention_rows_scratch_bytes(R, self.nh, self.kw, runs))
+        return runs, warps, 0, scratch, rt.tickets(R * self.nkv)
+
     def _decode_shape(self, ctx, capacity: int):
         """(runs, warps) for the decode kernel: each (row, kv head) is read by
         ``runs`` blocks of ``warps`` warps.  All of them should be resident at
@@ -544,16 +584,12 @@ class Attention:
         width = qkv.shape[1]
         cached = not (ctx.all_from_start and owns_cache)
         if cached and bf16 and native.attention_decode_supports(nh, nkv, hd, view.page_tokens):
-            splits, warps = self._decode_shape(ctx, ctx.cache.max_seq_len)
-            scratch = tickets = None
-            if splits > 1:
-                scratch = rt.scratch(native.attention_rows_scratch_bytes(R, nh, hd, splits))
-                tickets = rt.tickets(R * nkv)
+            splits, warps, slots, scratch, tickets = self._decode_launch(ctx)
             return native.attention_decode(qkv, width, view.k, view.v, view.page_table, view.page_tokens,
                                            view.ring_tokens, ctx.row_pos, ctx.row_seq, ctx.seq_slot, out,
                                            scratch, tickets, nh, nkv, hd, self.scale, 0.0, 0, splits, warps,
                                            fresh=ctx.max_count if rt.early_keys else 0, chunk=self.chunk,
-                                           sink=self.sink)
+                                           sink=self.sink, slots=slots)
         # the general kernel: the step's own keys from the packed rows, earlier ones from the cache
         splits = self._splits(ctx, ctx.cache.max_seq_len) if cached else 1
         scratch = None
@@ -734,17 +770,13 @@ class Attention:
             self._attend_pieces(qkv, out, ctx, view)
         elif qkv.dtype == torch.bfloat16 and native.attention_decode_supports(
                 nh, self.nkv, hd, view.page_tokens):
-            splits, warps = self._decode_shape(ctx, ctx.cache.max_seq_len)
-            scratch = tickets = None
-            if splits > 1:
-                scratch = rt.scratch(native.attention_rows_scratch_bytes(R, nh, hd, splits))
-                tickets = rt.tickets(R * self.nkv)
+            splits, warps, slots, scratch, tickets = self._decode_launch(ctx)
             native.attention_decode(qkv, width, view.k, view.v, view.page_table, view.page_tokens,
                                     view.ring_tokens, ctx.row_pos, ctx.row_seq, ctx.seq_slot, out,
                                     scratch, tickets, nh, self.nkv, hd, self.scale, self.softcap,
                                     self.window, splits, warps,
                                     fresh=ctx.max_count if rt.early_keys else 0, sink=self.sink,
-                                    keep=self.keep, fixed_tokens=view.fixed_tokens)
+                                    keep=self.keep, fixed_tokens=view.fixed_tokens, slots=slots)
         else:
             splits = self._splits(ctx, ctx.cache.max_seq_len)
             scratch = None

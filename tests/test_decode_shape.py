@@ -3,7 +3,7 @@ once, as few tiles of keys per warp as that allows, and no more warps than that 
 
 import itertools
 
-from strata_inference_b200.parts.attention import decode_shape
+from strata_inference_b200.parts.attention import decode_shape, shared_shape
 
 RES4, RES8 = 1776, 1184        # warps a device of 148 SMs holds: 3 blocks of 4, 1 block of 8 an SM
 
@@ -47,3 +47,19 @@ def test_few_rows_take_wide_blocks_and_one_tile_a_warp():
 def test_a_shape_the_wide_kernel_does_not_take():
     runs, warps = decode_shape(4, 8192, 0, RES4, 0)
     assert warps == 4 and runs >= 1
+
+
+def test_shared_blocks_are_resident_and_go_round():
+    for rows, n_kv, tiles in itertools.product((2, 3, 8, 33, 64, 111, 128), (1, 2, 4, 8, 16), (1, 7, 100, 512)):
+        shape = shared_shape(rows, n_kv, tiles, RES4)
+        if shape is None:           # not even blocks of one warp go round
+            assert RES4 // n_kv < rows
+            continue
+        slots, warps = shape
+        assert slots >= rows and warps in (1, 2, 4) and slots * warps * n_kv <= RES4
+
+
+def test_shared_blocks_are_wide_where_that_costs_no_tiles():
+    assert shared_shape(64, 4, 7, RES4) == (111, 4)         # short rows: one block each
+    assert shared_shape(64, 4, 188, RES4) == (222, 2)
+    assert shared_shape(100, 8, 257, RES4) == (222, 1)      # blocks of 2: hardly more than rows

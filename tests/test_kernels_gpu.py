@@ -228,6 +228,57 @@ def test_attention_decode_kernel(nh, nkv, hd, window, cap, splits, warps):
             _close(out[i].view(nh, hd), ref[r], dtype, f"decode rows together, row {r}")
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window,cap,slots,warps,picks", [
+    # as many blocks as rows; a block or two more; far more than there are tiles
+    (4, 2, 64, 0, 0.0, 5, 4, [2049, 0, 15, 16, 700]), (8, 4, 256, 0, 50.0, 7, 2, [2049, 31, 32, 1500, 999]),
+    (2, 2, 128, 0, 0.0, 400, 1, [100, 2049, 47]),
+    # one row's runs at the kernel's limit of 128
+    (8, 1, 128, 0, 0.0, 444, 1, [2049, 1, 16]),
+    # windows that begin inside a tile, with and without kept first positions, chunks
+    (8, 4, 256, 100, 50.0, 20, 2, [2049, 50, 99, 100, 115, 116]), (4, 1, 64, (70, 37), 0.0, 30, 4, [2049, 30, 70, 106, 107]),
+    (4, 2, 128, "chunk 100", 30.0, 9, 2, [2049, 99, 100, 199, 200, 0]),
+    # whole and part groups of 32 rows, the most rows there may be
+    (2, 1, 64, 0, 0.0, 150, 4, list(range(0, 2048, 64))), (2, 1, 64, 0, 0.0, 70, 2, list(range(5, 2050, 62))),
+    (2, 1, 64, 33, 0.0, 131, 1, list(range(2049, 1, -16)))])
+def test_attention_decode_shared_out(nh, nkv, hd, window, cap, slots, warps, picks):
+    """Blocks shared out by the rows' lengths: unequal rows in one launch against the plain
+    attention, a sink's weight among the denominator's terms."""
+    n = _native()
+    g = torch.Generator().manual_seed(29)
+    T, dtype, page = 2050, torch.bfloat16, 64
+    picks = picks[:128]
+    chunk, keep = 0, 0
+    if isinstance(window, str):
+        chunk, window = int(window.split()[1]), 0
+    elif isinstance(window, tuple):
+        window, keep = window
+    q = torch.randn(T, nh, hd, generator=g).to(dtype)
+    k = torch.randn(T, nkv, hd, generator=g).to(dtype)
+    v = torch.randn(T, nkv, hd, generator=g).to(dtype)
+    sink = torch.randn(nh, generator=g) + 2.0
+    scale = 3.0 / math.sqrt(hd)
+    kp, vp, table = _paged(k, v, page, 0, nkv, hd, dtype, range(T))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    R = len(picks)
+    tickets = torch.zeros(R * nkv, dtype=torch.int32, device=DEV)
+    out = torch.empty(R, nh * hd, dtype=dtype, device=DEV)
+    scratch = torch.empty(n.attention_rows_scratch_bytes(1, nh, hd, slots), dtype=torch.uint8, device=DEV)
+    qs = torch.stack([q[r].reshape(nh * hd) for r in picks]).contiguous().to(DEV)
+    n.attention_decode(qs, nh * hd, kp.to(DEV), vp.to(DEV), table.to(DEV), page, 0, i32(picks), i32([0] * R),
+                       i32([1]), out, scratch, tickets, nh, nkv, hd, scale, cap, window, 1, warps, chunk=chunk,
+                       sink=sink.to(DEV), keep=keep, slots=slots)
+    assert int(tickets.abs().sum()) == 0, "the ticket counters are put back"
+    for i, r in enumerate(picks):
+        pos = torch.arange(r + 1)
+        seen = (pos >= r - r % chunk) if chunk else (pos > r - window) | (pos < keep) if window else pos >= 0
+        s = torch.einsum("hd,thd->ht", q[r].double(), k[:r + 1].double().repeat_interleave(nh // nkv, 1)) * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        s = s.masked_fill(~seen, float("-inf"))
+        w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), 1)[:, :-1]
+        want = torch.einsum("ht,thd->hd", w, v[:r + 1].double().repeat_interleave(nh // nkv, 1))
+        _close(out[i].view(nh, hd), want, dtype, f"row {r}")
+
+
 @pytest.mark.parametrize("nh,nkv,hd,window,cap", [
     (4, 2, 64, 0, 0.0), (8, 4, 256, 100, 50.0), (4, 1, 128, 0, 30.0), (2, 2, 128, 70, 0.0),
     (8, 4, 256, 0, 0.0), (3, 3, 64, 17, 20.0)])
