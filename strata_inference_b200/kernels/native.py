@@ -53,6 +53,7 @@ def library():
     lib = ctypes.CDLL(path)
     lib.sib_last_error.restype = ctypes.c_char_p
     lib.sib_attention_rows_scratch_bytes.restype = c_longlong
+    lib.sib_chunked_scan_floats.restype = c_longlong
     if lib.sib_compiled_arch() != 100:
         raise KernelError(f"{path} was not compiled for sm_100a")
     _lib = lib
@@ -1191,6 +1192,27 @@ def _scan_work(kind, rows, n_seqs, n_heads, key_dim, cols):
         7.0 * rows * n_heads * key_dim * cols
 
 
+# A step whose longest sequence has at least this many rows walks them in chunks (csrc/chunked_scan.cu)
+# instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us one by one and 76 in chunks, 300
+# rows 94 and 60 (4 heads of 64 x 64).
+CHUNKED_SCAN_MIN_ROWS = 160
+# ... unless the chunks' scratch memory would come to more 32-bit floats than this
+CHUNKED_SCAN_MAX_FLOATS = 1 << 29
+
+
+def chunked_scan_scratch(out: torch.Tensor, ctx, n_heads: int, key_dim: int, cols: int, delta: bool = False,
+                         memory: bool = False) -> Optional[torch.Tensor]:
+    """Scratch memory of a scan in chunks; None where the scan goes row by row: no sequence of the
+    step is long enough, the kernel does not take the key width, or it would need too much."""
+    if ctx.max_count < CHUNKED_SCAN_MIN_ROWS:
+        return None
+    n = library().sib_chunked_scan_floats(c_longlong(out.shape[0]), c_int(n_heads), c_int(key_dim), c_int(cols),
+                                          c_int(1 if delta else 0), c_int(1 if memory else 0))
+    if not 0 < n <= CHUNKED_SCAN_MAX_FLOATS:
+        return None
+    return torch.empty(n, dtype=torch.float32, device=out.device)
+
+
 @_timed(lambda qn, kn, vc, decay, beta, state, out, ctx, n_heads, n_kv, key_dim, value_dim: _scan_work(
     "delta_scan", out.shape[0], ctx.n_seqs, n_heads, key_dim, value_dim))
 def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torch.Tensor,
@@ -1204,6 +1226,14 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torc
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("delta_scan: the state is too small for the matrices")
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim, delta=True)
+    if scratch is not None:
+        _check(library().sib_delta_scan_chunked(
+            _ptr(qn), _ptr(kn), _ptr(vc), _ptr(decay), _ptr(beta), _ptr(state),
+            c_longlong(state.stride(0)), _ptr(out), _ptr(scratch), _ptr(ctx.seq_slot), _ptr(ctx.seq_start),
+            _ptr(ctx.seq_end), _ptr(ctx.seq_row0), c_int(rows), c_int(ctx.n_seqs), c_int(ctx.max_count),
+            c_int(n_heads), c_int(n_kv), c_int(key_dim), c_int(value_dim), _stream()))
+        return out
     _check(library().sib_delta_scan(
         _ptr(qn), _ptr(kn), _ptr(vc), _ptr(decay), _ptr(beta), _ptr(state),
         c_longlong(state.stride(0)), _ptr(out), _ptr(ctx.seq_slot), _ptr(ctx.seq_start),
@@ -1233,6 +1263,15 @@ def memory_scan(proj: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, 
     _f32(m_out, rows * n_heads, "m_out")
     if state.shape[1] < n_heads * (value_dim + 1) * key_dim + n_heads:
         raise KernelError("memory_scan: the state is too small")
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim + 1, memory=True)
+    if scratch is not None:
+        _check(library().sib_memory_scan_chunked(
+            _ptr(proj), c_longlong(proj.stride(0)), _code(proj.dtype), c_longlong(2 * nq + 2 * nv),
+            c_longlong(2 * nq + 2 * nv + n_heads), _ptr(bias_i), _ptr(bias_f), c_float(cap), _ptr(state),
+            c_longlong(state.stride(0)), _ptr(out), _ptr(m_out), _ptr(scratch), _ptr(ctx.seq_slot),
+            _ptr(ctx.seq_start), _ptr(ctx.seq_end), _ptr(ctx.seq_row0), c_int(rows), c_int(ctx.n_seqs),
+            c_int(ctx.max_count), c_int(n_heads), c_int(key_dim), c_int(value_dim), _stream()))
+        return out
     _check(library().sib_memory_scan(
         _ptr(proj), c_longlong(proj.stride(0)), _code(proj.dtype), c_longlong(2 * nq + 2 * nv),
         c_longlong(2 * nq + 2 * nv + n_heads), _ptr(bias_i), _ptr(bias_f), c_float(cap), _ptr(state),
@@ -1283,6 +1322,16 @@ def retention_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: 
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("retention_scan: the state is too small for the matrices")
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim)
+    if scratch is not None:
+        nq, nv = n_heads * key_dim, n_heads * value_dim
+        _check(library().sib_gated_scan_chunked(
+            _ptr(qn), _ptr(kn), _ptr(vc), c_longlong(nq), c_longlong(nq), c_longlong(nv), None, None,
+            _ptr(decay), _ptr(state), c_longlong(state.stride(0)), _ptr(out), _ptr(scratch),
+            _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_end), _ptr(ctx.seq_row0), c_int(rows),
+            c_int(ctx.n_seqs), c_int(ctx.max_count), c_int(n_heads), c_int(n_heads), c_int(key_dim),
+            c_int(value_dim), _stream()))
+        return out
     _check(library().sib_retention_scan(
         _ptr(qn), _ptr(kn), _ptr(vc), _ptr(decay), _ptr(state), c_longlong(state.stride(0)),
         _ptr(out), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_end), _ptr(ctx.seq_row0),
@@ -1340,6 +1389,15 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, keep: torch.Te
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("gated_scan: the state is too small for the matrices")
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim)
+    if scratch is not None:
+        _check(library().sib_gated_scan_chunked(
+            _ptr(q), _ptr(k), _ptr(v), c_longlong(q.stride(0)), c_longlong(k.stride(0)),
+            c_longlong(v.stride(0)), _ptr(keep), _ptr(take), None, _ptr(state), c_longlong(state.stride(0)),
+            _ptr(out), _ptr(scratch), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_end),
+            _ptr(ctx.seq_row0), c_int(rows), c_int(ctx.n_seqs), c_int(ctx.max_count), c_int(n_heads),
+            c_int(n_kv), c_int(key_dim), c_int(value_dim), _stream()))
+        return out
     _check(library().sib_gated_scan(
         _ptr(q), _ptr(k), _ptr(v), c_longlong(q.stride(0)), c_longlong(k.stride(0)),
         c_longlong(v.stride(0)), _ptr(keep), _ptr(take), _ptr(state), c_longlong(state.stride(0)),
