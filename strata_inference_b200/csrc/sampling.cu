@@ -23,8 +23,11 @@
 // 4 bits a pass (16 buckets of count and mass per pass, 8 passes a search).
 // All sums are taken in a fixed order, so a draw is reproducible.
 // With top-k on and few candidates (at most SAMPLE_LIST at or above the k-th key, ties
-// included) only the first of the three searches runs, without masses; the candidates are
-// gathered into a list, sorted and walked one after the other (sample_from_short_list).
+// included) the candidates are gathered into a list, sorted and walked one after the other
+// (sample_from_short_list).  What to gather is known without a search through the row: the
+// threads' maxima of the first pass are so many different elements, so the k-th largest of
+// them is at most the row's k-th largest element (floor_of_maxima), and the elements above it are
+// hardly more than k.  Only where they are too many does the first of the three searches run.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -34,6 +37,7 @@ namespace cg = cooperative_groups;
 #define SAMPLE_CLUSTER 8
 #define SAMPLE_THREADS 512
 #define SAMPLE_WARPS (SAMPLE_THREADS / 32)
+#define SAMPLE_BATCH 8      // elements a thread asks for at once in a pass without masses
 #define SAMPLE_LIST 256     // a top-k set of at most this many candidates is sorted and walked as a list
 
 __device__ __forceinline__ uint32_t order_key(float z) {
@@ -258,6 +262,38 @@ __device__ Crossing find_crossing(Cluster& c, const float* row, int lo, int hi, 
     return r;
 }
 
+// A key that at least `top_k` of the row's elements reach: the lowest key of the first bucket, 4 bits
+// a pass, at which the running count of the threads' maxima (`mine`, one a thread; `some`: it has one)
+// reaches `top_k`.  The walk stops as soon as few maxima reach the bucket.  False: there are fewer
+// maxima than `top_k`.
+__device__ bool floor_of_maxima(Cluster& c, uint32_t mine, bool some, int top_k, uint32_t* floor_key) {
+    SampleShared* sh = c.sh;
+    uint32_t path = 0;
+    int above = 0;
+    for (int level = 0; level < 8; ++level) {
+        const int shift = 28 - 4 * level;
+        const uint32_t path_mask = level == 0 ? 0u : (0xffffffffu << (shift + 4));
+        const bool in = some && (mine & path_mask) == (path & path_mask);
+#pragma unroll
+        for (int b = 0; b < 16; ++b) {
+            sh->bins_f[b][threadIdx.x] = 0.f;
+            sh->bins_i[b][threadIdx.x] = in && (int)((mine >> shift) & 15u) == b ? 1 : 0;
+        }
+        cluster_bucket_totals(c);
+        int pick = -1, upto = above;
+        for (int b = 15; b >= 0 && pick < 0; --b) {
+            upto += sh->tot_i[b];
+            if (upto >= top_k) pick = b;
+            else above = upto;
+        }
+        if (pick < 0) return false;          // (in the first pass only)
+        path |= (uint32_t)pick << shift;
+        if (upto <= SAMPLE_LIST / 2) break;
+    }
+    *floor_key = path;
+    return true;
+}
+
 // Publish one integer per block (one block holds a value >= 0, the others -1) and
 // return that value in every block (-1 if nobody had one).
 __device__ int cluster_share_found(Cluster& c, int found) {
@@ -324,20 +360,40 @@ __device__ int nth_with_key(Cluster& c, const float* row, int lo, int hi, float 
 // (-1 elsewhere); the caller shares it.
 __device__ int sample_from_short_list(Cluster& c, const float* row, int lo, int hi, float inv_t,
                                       float zmax, uint32_t floor_key, int top_k, float top_p,
-                                      float r, int fallback, float whole_mass = -1.f) {
+                                      float r, int fallback, float whole_mass = -1.f,
+                                      bool* too_many = nullptr) {
     SampleShared* sh = c.sh;
-    for (int i = lo + threadIdx.x; i < hi; i += SAMPLE_THREADS) {
-        const float z = row[i] * inv_t;
-        if (order_key(z) >= floor_key) {
-            const int slot = atomicAdd(&c.first->list_n, 1);
-            if (slot < SAMPLE_LIST) {
-                c.first->list_z[slot] = z;
-                c.first->list_i[slot] = i;
+    for (int i0 = lo + threadIdx.x; i0 < hi; i0 += SAMPLE_BATCH * SAMPLE_THREADS) {
+        float v[SAMPLE_BATCH];
+#pragma unroll
+        for (int k = 0; k < SAMPLE_BATCH; ++k) {
+            const int i = i0 + k * SAMPLE_THREADS;
+            v[k] = i < hi ? row[i] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < SAMPLE_BATCH; ++k) {
+            const int i = i0 + k * SAMPLE_THREADS;
+            const float z = v[k] * inv_t;
+            if (i < hi && order_key(z) >= floor_key) {
+                const int slot = atomicAdd(&c.first->list_n, 1);
+                if (slot < SAMPLE_LIST) {
+                    c.first->list_z[slot] = z;
+                    c.first->list_i[slot] = i;
+                }
             }
         }
     }
     c.g.sync();
     int token = -1;
+    if (too_many) {              // (the caller can do without the list)
+        *too_many = c.first->list_n > SAMPLE_LIST;
+        if (*too_many) {
+            c.g.sync();          // everyone has read the count
+            if (c.rank == 0 && threadIdx.x == 0) sh->list_n = 0;
+            c.g.sync();
+            return token;
+        }
+    }
     if (c.rank == 0) {
         const int n = min(sh->list_n, SAMPLE_LIST);
         if ((int)threadIdx.x < n) {
@@ -391,7 +447,9 @@ __device__ int sample_from_short_list(Cluster& c, const float* row, int lo, int 
     return token;
 }
 
-__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS)
+// (two blocks an SM: with one, which is what the registers of a build without a bound leave, 64 rows of the
+// cluster of 8 are four waves)
+__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, 2)
 sample_rows_kernel(SampleArgs p) {
     extern __shared__ __align__(16) unsigned char sample_smem[];
     SampleShared* sh = reinterpret_cast<SampleShared*>(sample_smem);
@@ -413,10 +471,19 @@ sample_rows_kernel(SampleArgs p) {
     // ---- the maximum and its first index ----
     float best = -INFINITY;
     int best_i = 0x7fffffff;
-    for (int i = lo + threadIdx.x; i < hi; i += SAMPLE_THREADS) {
-        const float v = row[i];
-        if (v > best) { best = v; best_i = i; }     // ascending i per thread: first maximum
+    for (int i0 = lo + threadIdx.x; i0 < hi; i0 += SAMPLE_BATCH * SAMPLE_THREADS) {
+        float v[SAMPLE_BATCH];
+#pragma unroll
+        for (int k = 0; k < SAMPLE_BATCH; ++k) {
+            const int i = i0 + k * SAMPLE_THREADS;
+            v[k] = i < hi ? row[i] : -INFINITY;
+        }
+#pragma unroll
+        for (int k = 0; k < SAMPLE_BATCH; ++k)
+            if (v[k] > best) { best = v[k]; best_i = i0 + k * SAMPLE_THREADS; }   // ascending i per thread: first maximum
     }
+    const float own_best = best;
+    const bool own_some = best_i != 0x7fffffff;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -524,7 +591,19 @@ sample_rows_kernel(SampleArgs p) {
     } else {
         Kept kept{0u, 0, 0.f};
         bool listed = false;
-        if (use_k) {
+        uint32_t floor_key;
+        if (use_k && p.top_k <= SAMPLE_LIST / 2 &&
+            floor_of_maxima(c, order_key(own_best * inv_t), own_some, p.top_k, &floor_key)) {
+            bool too_many;
+            token = sample_from_short_list(c, row, lo, hi, inv_t, zmax, floor_key, p.top_k, p.top_p, r,
+                                           best_i, -1.f, &too_many);
+            if (!too_many) {
+                listed = true;
+                token = cluster_share_found(c, token);
+                if (token < 0) token = best_i;
+            }
+        }
+        if (use_k && !listed) {
             // (the search for the k-th largest counts only: no masses are summed)
             // (and it stops as soon as the bucket it has come to, with everything above it,
             // fits the list: the list is sorted anyway)

@@ -997,6 +997,36 @@ def test_sampling_with_ties_at_the_edge_of_top_k(n_top, top_k, top_p):
     assert differ <= 2, f"{differ} of {2 * draws} draws differ from the plain sampler"
 
 
+@pytest.mark.parametrize("vocab,top_k,top_p", [
+    (3, 2, 1.0), (4096, 128, 1.0), (4097, 129, 0.9), (30000, 40, 0.95), (30000, 1, 1.0), (30000, 127, 0.8)])
+@pytest.mark.parametrize("place", ["spread", "one thread", "one block", "few finite"])
+def test_sampling_of_the_top_k_wherever_they_lie(vocab, top_k, top_p, place):
+    """The threads' maxima bound the k-th largest logit well where the largest are spread over the threads
+    and badly where one thread holds them all (then everything above the bound does not fit the
+    list); with fewer finite logits than top-k there is no bound."""
+    n = _native()
+    g = torch.Generator().manual_seed(31)
+    logits = torch.randn(vocab, generator=g)
+    per_block = -(-vocab // 8)
+    if place == "one thread":            # a thread's elements lie 512 apart in its block's eighth
+        at = torch.arange(vocab)[per_block * 3 + 5:per_block * 4:512]
+    else:
+        at = torch.arange(vocab)[per_block * 5:per_block * 6]
+    if place != "spread" and at.numel():
+        logits[at] = 5.0 + torch.randn(at.numel(), generator=g)
+    if place == "few finite":
+        logits[:] = -math.inf
+        logits[torch.randperm(vocab, generator=g)[:max(1, top_k // 2)]] = torch.randn(max(1, top_k // 2), generator=g)
+    dev = logits[None].to(DEV)
+    state = torch.tensor([77], dtype=torch.int64, device=DEV)
+    out = torch.empty(1, dtype=torch.int32, device=DEV)
+    rng, differ = plain.XorShift64(77), 0
+    for _ in range(20):
+        n.sample_rows(dev, 0.9, top_k, top_p, state, out)
+        differ += plain.sample_token(logits, 0.9, top_k, top_p, rng) != int(out)
+    assert differ <= 1, f"{differ} of 20 draws differ from the plain sampler"
+
+
 def test_sampling_at_the_vocabulary_of_the_real_model():
     n = _native()
     g = torch.Generator().manual_seed(10)
