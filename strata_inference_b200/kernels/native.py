@@ -1638,6 +1638,38 @@ def attention_decode_resident_warps(n_heads: int, n_kv: int, head_dim: int, warp
                                                                 c_int(head_dim), c_int(warps)))
 
 
+# 32-bit prompts whose longest has at least this many rows go to the tiled kernel
+ATTENTION_PROMPT_F32_MIN_ROWS = 2
+
+
+def attention_prompt_f32_supports(n_heads: int, n_kv: int, head_dim: int) -> bool:
+    return bool(library().sib_attention_prompt_f32_supports(c_int(n_heads), c_int(n_kv), c_int(head_dim)))
+
+
+@_timed(lambda qkv, out, ctx, n_heads, n_kv, head_dim, *a, **kw: (
+    "attention_prompt_f32", 2 * _nbytes(out) * (1 + 2 * n_kv / n_heads),
+    2.0 * (ctx.row_pos.to(torch.int64) + 1).sum().item() * 2 * n_heads * head_dim))
+def attention_prompt_f32(qkv: torch.Tensor, out: torch.Tensor, ctx, n_heads: int, n_kv: int, head_dim: int,
+                         scale: float, softcap: float, window: int, chunk: int = 0, keep: int = 0,
+                         sink: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Attention of packed 32-bit prompts ``[q | k | v]`` that start at position 0 over their own keys and
+    values (csrc/attention_prompt_f32.cu); options as of ``attention_rows``."""
+    _want(qkv, torch.float32, "qkv", contiguous=False)
+    _want(out, torch.float32, "out")
+    if qkv.stride(1) != 1 or qkv.shape[1] < (n_heads + 2 * n_kv) * head_dim or out.shape[0] != qkv.shape[0]:
+        raise KernelError("attention_prompt_f32: rows of q | k | v and as many rows of the output are needed")
+    if sink is not None:
+        _f32(sink, n_heads, "sink")
+    q = qkv.data_ptr()
+    k = q + 4 * n_heads * head_dim
+    _check(library().sib_attention_prompt_f32(
+        c_void_p(q), c_int(qkv.stride(0)), c_void_p(k), c_void_p(k + 4 * n_kv * head_dim), c_int(qkv.stride(0)),
+        _ptr(ctx.seq_start), _ptr(ctx.seq_end), _ptr(ctx.seq_row0), _ptr(out), c_int(ctx.n_seqs),
+        c_int(ctx.max_count), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_float(scale), c_float(softcap),
+        c_int(window), c_int(chunk), c_int(keep), _ptr(sink), _stream()))
+    return out
+
+
 @_timed(lambda q, q_stride, k_pool, v_pool, page_table, page_tokens, ring_tokens, row_pos, row_seq,
         seq_slot, out, scratch, tickets, n_heads, n_kv, head_dim, scale, softcap, window, splits,
         warps=4, fresh=0, chunk=0, sink=None, keep=0, fixed_tokens=0, slots=0: _attention_cache_work(

@@ -590,6 +590,10 @@ class Attention:
                                            scratch, tickets, nh, nkv, hd, self.scale, 0.0, 0, splits, warps,
                                            fresh=ctx.max_count if rt.early_keys else 0, chunk=self.chunk,
                                            sink=self.sink, slots=slots)
+        if (prompts and not bf16 and owns_cache and ctx.max_count >= native.ATTENTION_PROMPT_F32_MIN_ROWS
+                and native.attention_prompt_f32_supports(nh, nkv, hd)):
+            return native.attention_prompt_f32(qkv, out, ctx, nh, nkv, hd, self.scale, 0.0, 0, chunk=self.chunk,
+                                               sink=self.sink)
         # the general kernel: the step's own keys from the packed rows, earlier ones from the cache
         splits = self._splits(ctx, ctx.cache.max_seq_len) if cached else 1
         scratch = None
@@ -755,6 +759,10 @@ class Attention:
             native.attention_prefill(qkv, out, ctx.seq_row0, ctx.seq_end, ctx.n_seqs,
                                      ctx.max_count, nh, self.nkv, hd, self.scale, self.softcap,
                                      self.window, self.keep, self.sink, self.exact_cap)
+        elif fresh and qkv.dtype == torch.float32 and ctx.max_count >= native.ATTENTION_PROMPT_F32_MIN_ROWS \
+                and native.attention_prompt_f32_supports(nh, self.nkv, hd):
+            native.attention_prompt_f32(qkv, out, ctx, nh, self.nkv, hd, self.scale, self.softcap, self.window,
+                                        keep=self.keep, sink=self.sink)
         elif fresh:
             k_new = qkv[:, nh * hd:]
             v_new = qkv[:, (nh + nkv) * hd:]
