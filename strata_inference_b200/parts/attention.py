@@ -422,10 +422,11 @@ class Attention:
         runs, warps = self._decode_shape(ctx, ctx.cache.max_seq_len)
         # (few (row, kv head) pairs have many runs each, and joining those costs more than unequal
         # lengths do: 5 rows of 100 to 5 000 positions and one kv head take 12 us with blocks of 8
-        # warps, 27 shared out)
-        if warps < 8 and 1 < R <= native.attention_decode_max_shared_rows():
-            shared = shared_shape(R, self.nkv, -(-self._longest(ctx, ctx.cache.max_seq_len) // 16),
-                                  self._resident_warps[4])
+        # warps, 27 shared out.  Where a warp walks two tiles at most anyway there is nothing to share:
+        # 8 rows of up to 1 088 seen positions, 8 kv heads of 128, take 10.6 us either way)
+        tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
+        if warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
+            shared = shared_shape(R, self.nkv, tiles, self._resident_warps[4])
             if shared is not None:
                 slots, warps = shared
                 scratch = rt.scratch(native.attention_rows_scratch_bytes(1, self.nh, self.kw, slots))
