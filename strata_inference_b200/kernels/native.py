@@ -1193,8 +1193,8 @@ def _scan_work(kind, rows, n_seqs, n_heads, key_dim, cols):
 
 
 # A step whose longest sequence has at least this many rows walks them in chunks (csrc/chunked_scan.cu)
-# instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us one by one and 76 in chunks, 300
-# rows 94 and 60 (4 heads of 64 x 64).
+# instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us one by one and 83 in chunks, 300
+# rows 95 and 60 (4 heads of 64 x 64).
 CHUNKED_SCAN_MIN_ROWS = 160
 # ... unless the chunks' scratch memory would come to more 32-bit floats than this
 CHUNKED_SCAN_MAX_FLOATS = 1 << 29
@@ -1206,8 +1206,8 @@ def chunked_scan_scratch(out: torch.Tensor, ctx, n_heads: int, key_dim: int, col
     step is long enough, the kernel does not take the key width, or it would need too much."""
     if ctx.max_count < CHUNKED_SCAN_MIN_ROWS:
         return None
-    n = library().sib_chunked_scan_floats(c_longlong(out.shape[0]), c_int(n_heads), c_int(key_dim), c_int(cols),
-                                          c_int(1 if delta else 0), c_int(1 if memory else 0))
+    n = library().sib_chunked_scan_floats(c_longlong(out.shape[0]), c_int(ctx.n_seqs), c_int(n_heads), c_int(key_dim),
+                                          c_int(cols), c_int(1 if delta else 0), c_int(1 if memory else 0))
     if not 0 < n <= CHUNKED_SCAN_MAX_FLOATS:
         return None
     return torch.empty(n, dtype=torch.float32, device=out.device)
