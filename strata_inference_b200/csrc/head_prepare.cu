@@ -385,12 +385,46 @@ __global__ void head_gate_kernel(const T* __restrict__ o, const T* __restrict__ 
     }
 }
 
+// The same for bfloat16 heads whose widths are multiples of 8: a thread takes 8 neighbouring elements, 16
+// bytes at a time, and makes their gate once.  (2 048 rows of 8 heads of 256: element by element, an
+// exponential and two divisions of indices each, 17.7 us; so 4.4.)
+__global__ void __launch_bounds__(256)
+head_gate8_kernel(const __nv_bfloat16* o, const __nv_bfloat16* gate, long long gate_stride, __nv_bfloat16* y,
+                  int n_heads, int vd, int pad, size_t total8) {
+    pdl_trigger();
+    pdl_wait();
+    const int per_head = vd / 8, per_row = n_heads * per_head;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total8;
+         idx += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = idx / per_row;
+        const int rest = (int)(idx - r * per_row), h = rest / per_head, e = 8 * (rest - h * per_head);
+        const uint4 a = *reinterpret_cast<const uint4*>(o + (r * n_heads + h) * (size_t)pad + e);
+        const float g = gate ? 1.0f / (1.0f + expf(-to_f32(gate[r * gate_stride + h]))) : 1.0f;
+        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+        uint32_t out[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(w[i] << 16) * g,
+                                                            __uint_as_float(w[i] & 0xffff0000u) * g);
+            out[i] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        *reinterpret_cast<uint4*>(y + 8 * idx) = make_uint4(out[0], out[1], out[2], out[3]);
+    }
+}
+
 SIB_EXPORT int sib_head_gate(const void* o, const void* gate, long long gate_stride, void* y,
                              int dtype, int rows, int n_heads, int vd, int pad, void* stream) {
     if (rows == 0) return 0;
     SIB_REQUIRE(rows > 0 && n_heads > 0 && vd > 0 && pad >= vd,
                 "head_gate: rows=%d heads=%d width=%d of %d", rows, n_heads, vd, pad);
     const size_t total = (size_t)rows * n_heads * vd;
+    if (dtype == SIB_BF16 && vd % 8 == 0 && pad % 8 == 0 && ((uintptr_t)o % 16) == 0 && ((uintptr_t)y % 16) == 0) {
+        const size_t want8 = (total / 8 + 255) / 256;
+        sib_launch_chained(head_gate8_kernel, dim3((unsigned)(want8 < 148 * 16 ? want8 : 148 * 16)), dim3(256), 0,
+                           (cudaStream_t)stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)gate, gate_stride,
+                           (__nv_bfloat16*)y, n_heads, vd, pad, total / 8);
+        return sib_check_launch("head_gate");
+    }
     const size_t want = (total + 255) / 256;
     const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
     SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(head_gate_kernel<T>, dim3(blocks), dim3(256), 0,

@@ -578,6 +578,62 @@ __global__ void routed_combine_kernel(const T* __restrict__ ys, const int* __res
     }
 }
 
+// The same for bfloat16 rows whose width is a multiple of 8: a thread takes 8 neighbouring columns, 16 bytes at
+// a time, all of its pairs' loads (up to 8) ahead of the sums, which are those above.  (3 300 rows of
+// 2 048, 4 experts each: column by column 37 us, so 14.6, 12 at the copy bandwidth.)
+__global__ void __launch_bounds__(256)
+routed_combine8_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ where,
+                       const float* __restrict__ weights, const __nv_bfloat16* __restrict__ base,
+                       const float* __restrict__ base_weight, __nv_bfloat16* __restrict__ out, int width, int top,
+                       size_t total8) {
+    constexpr int AHEAD = 8;
+    pdl_trigger();
+    pdl_wait();
+    const int per_row = width / 8;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / per_row;
+        const int n = 8 * (int)(i - r * per_row);
+        float acc[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+        if (base) {
+            const uint4 v = reinterpret_cast<const uint4*>(base)[i];
+            const float bw = base_weight ? base_weight[r] : 1.0f;
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[2 * e] = __uint_as_float(w[e] << 16) * bw;
+                acc[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u) * bw;
+            }
+        }
+        for (int k0 = 0; k0 < top; k0 += AHEAD) {
+            uint4 v[AHEAD];
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k)
+                if (k0 + k < top)
+                    v[k] = *reinterpret_cast<const uint4*>(ys + (size_t)where[r * top + k0 + k] * width + n);
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                if (k0 + k >= top) break;
+                const float pw = weights ? weights[r * top + k0 + k] : 1.0f;
+                const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    acc[2 * e] += pw * __uint_as_float(w[e] << 16);
+                    acc[2 * e + 1] += pw * __uint_as_float(w[e] & 0xffff0000u);
+                }
+            }
+        }
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1]);
+            o[e] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        reinterpret_cast<uint4*>(out)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 int grid_for(size_t total) {
     const size_t want = (total + 255) / 256;
     return (int)(want < 148 * 16 ? (want ? want : 1) : 148 * 16);
@@ -745,6 +801,13 @@ SIB_EXPORT int sib_routed_combine(const void* ys, const int* where, const float*
     SIB_REQUIRE(rows > 0 && width > 0 && top > 0, "routed_combine: rows=%d width=%d top=%d", rows,
                 width, top);
     const size_t total = (size_t)rows * width;
+    if (dtype == SIB_BF16 && width % 8 == 0 && ((uintptr_t)ys % 16) == 0 && ((uintptr_t)base % 16) == 0 &&
+        ((uintptr_t)out % 16) == 0) {
+        sib_launch_chained(routed_combine8_kernel, dim3(grid_for(total / 8)), dim3(256), 0, (cudaStream_t)stream,
+                           (const __nv_bfloat16*)ys, where, weights, (const __nv_bfloat16*)base, base_weight,
+                           (__nv_bfloat16*)out, width, top, total / 8);
+        return sib_check_launch("routed_combine");
+    }
     SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(routed_combine_kernel<T>, dim3(grid_for(total)),
                                                  dim3(256), 0, (cudaStream_t)stream, (const T*)ys,
                                                  where, weights, (const T*)base, base_weight, (T*)out, width,
