@@ -146,14 +146,15 @@ __device__ __forceinline__ void skinny_linear_body(
     const uint4 zero = make_uint4(0, 0, 0, 0);
 
     // The weights do not depend on the kernel before this one: pull this block's towards L2 while
-    // that kernel is still running, then wait for it.  A block that has its rows to itself asks for
-    // its runs of 8 rows, which are contiguous, as a whole, and for those of the block that takes its
-    // place on the SM: else the memory idles between the first blocks' last loads and the next ones'
-    // first.  (Gemma2-2B shape, batch 1: gate/up product, 1 152 blocks of which 592 are resident, 16.5 ->
-    // 14.4 us, logits 188 -> 177 us.)  The blocks of a cluster ask line by line for their own runs of
-    // k (runs of rows instead: output product 4.5 -> 7 us).
+    // that kernel is still running, then wait for it.  Where there are more blocks than the device
+    // holds, a block asks for its runs of 8 rows, which are contiguous, as a whole, and for those of the
+    // block that takes its place on the SM: else the memory idles between the first blocks' last
+    // loads and the next ones' first.  (Gemma2-2B shape, batch 1: gate/up product, 1 152 blocks of which
+    // 592 are resident, 16.5 -> 14.4 us, logits 188 -> 177 us.)  Blocks that are all resident ask line by
+    // line for their own runs of k, in the order they will read them (rows as a whole instead:
+    // output product 4.5 -> 7 us, a step with 8 192 x 2 048 products 1 % slower).
     pdl_trigger();
-    if (ksplit > 1 || K > 32768) {
+    if (EPI == EPI_ROPE || ahead == 0 || K > 32768) {
         if (t == 0) {
             for (int kb = (rank * 8 + warp) * 64; kb < K; kb += ksplit * 8 * 64) {
 #pragma unroll
@@ -164,9 +165,9 @@ __device__ __forceinline__ void skinny_linear_body(
             }
         }
     } else if (threadIdx.x < 2 * MT) {
-        const int run = (threadIdx.x & 1 ? run_b : run_a) + 16 * (threadIdx.x >> 1);
+        const int run = n0 + 8 * (int)threadIdx.x, next = run + ahead * 16 * MT;
         prefetch_rows(W, run, min(run + 8, N), K);
-        if (EPI != EPI_ROPE && ahead > 0) prefetch_rows(W, run + ahead * 16 * MT, min(run + ahead * 16 * MT + 8, N), K);
+        prefetch_rows(W, next, min(next + 8, N), K);
     }
     pdl_wait();
 
@@ -386,7 +387,9 @@ static int launch_skinny(const void* W, const void* x, void* y, int R, int N, in
         if (!per_sm && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, skinny_linear_kernel<NT, MT, OutT, EPI>, 256,
                                                                      smem) != cudaSuccess)
             per_sm = 1;
-        if (blocks > per_sm * sms) ahead = per_sm * sms;
+        // (what all blocks ask for ahead has to stay in L2 beside what they read: 44 MB at a width of 2 304; at
+        // 3 584 it would be 68 MB of 126, and the logits of that width took 80 us more with it)
+        if (blocks > per_sm * sms && (long long)per_sm * sms * 16 * MT * K * 2 <= (48ll << 20)) ahead = per_sm * sms;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks, ksplit, 1);
