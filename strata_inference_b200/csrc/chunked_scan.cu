@@ -819,43 +819,55 @@ template <typename T> __global__ void __launch_bounds__(32) memory_gates_kernel(
     float m = cell ? *cell : 0.f;
     const T* gi = (const T*)p.gate_i + h;
     const T* gf = (const T*)p.gate_f + h;
-    T ri = from_f32<T>(0.f), rf = ri;
-    auto fetch = [&](int t) {
-        if (t < n) {
-            ri = gi[(row0 + t) * p.stride];
-            rf = gf[(row0 + t) * p.stride];
-        }
-    };
-    fetch(lane);
-    for (int t0 = 0; t0 < n; t0 += 32) {
-        const int t = t0 + lane;
-        float i = p.cap * tanhf((to_f32(ri) + bias_i) / p.cap);
-        float f = p.cap * tanhf((to_f32(rf) + bias_f) / p.cap);
-        f = -(fmaxf(-f, 0.f) + log1pf(expf(-fabsf(f))));      // log sigmoid
-        if (t >= n) {
-            i = -INFINITY;
-            f = 0.f;
-        }
-        fetch(t + 32);
-        float F = f, M = i;
+    // (the gates' inputs of AHEAD groups are asked for while the AHEAD before them are worked on)
+    constexpr int AHEAD = 4;
+    T ri[AHEAD], rf[AHEAD];
+    auto fetch = [&](int t0) {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float F1 = __shfl_up_sync(0xffffffffu, F, o), M1 = __shfl_up_sync(0xffffffffu, M, o);
-            if (lane >= o) {
-                M = fmaxf(M1 + F, M);
-                F += F1;
+        for (int i = 0; i < AHEAD; ++i) {
+            const int t = t0 + 32 * i + lane;
+            ri[i] = rf[i] = from_f32<T>(0.f);
+            if (t < n) {
+                ri[i] = gi[(row0 + t) * p.stride];
+                rf[i] = gf[(row0 + t) * p.stride];
             }
         }
-        const float now = fmaxf(F + m, M);
-        float before = __shfl_up_sync(0xffffffffu, now, 1);
-        if (lane == 0) before = m;
-        if (t < n) {
-            const size_t at = (row0 + t) * p.H + h;
-            p.keep[at] = expf(f + before - now);
-            p.take[at] = expf(i - now);
-            p.m_out[at] = now;
+    };
+    fetch(0);
+    for (int t00 = 0; t00 < n; t00 += 32 * AHEAD) {
+        float gate[AHEAD], forget[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            const int t = t00 + 32 * k + lane;
+            const float z = p.cap * tanhf((to_f32(rf[k]) + bias_f) / p.cap);
+            gate[k] = t < n ? p.cap * tanhf((to_f32(ri[k]) + bias_i) / p.cap) : -INFINITY;
+            forget[k] = t < n ? -(fmaxf(-z, 0.f) + log1pf(expf(-fabsf(z)))) : 0.f;      // log sigmoid
         }
-        m = __shfl_sync(0xffffffffu, now, 31);
+        fetch(t00 + 32 * AHEAD);
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            const int t = t00 + 32 * k + lane;
+            const float i = gate[k], f = forget[k];
+            float F = f, M = i;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float F1 = __shfl_up_sync(0xffffffffu, F, o), M1 = __shfl_up_sync(0xffffffffu, M, o);
+                if (lane >= o) {
+                    M = fmaxf(M1 + F, M);
+                    F += F1;
+                }
+            }
+            const float now = fmaxf(F + m, M);
+            float before = __shfl_up_sync(0xffffffffu, now, 1);
+            if (lane == 0) before = m;
+            if (t < n) {
+                const size_t at = (row0 + t) * p.H + h;
+                p.keep[at] = expf(f + before - now);
+                p.take[at] = expf(i - now);
+                p.m_out[at] = now;
+            }
+            m = __shfl_sync(0xffffffffu, now, 31);
+        }
     }
     if (cell && lane == 0) *cell = m;
 }

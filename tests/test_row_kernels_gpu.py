@@ -72,3 +72,63 @@ def test_head_norm_gate(rows, heads, vd, memory, act):
     want = (x * (torch.sigmoid(a) if act else a * torch.sigmoid(a))).reshape(rows, -1)
     # (a sum of vd squares, two divisions, a root and an exponential)
     assert bool(((y.double().cpu() - want).abs() <= (vd + 16) * 2.0 ** -24 * want.abs() + 1e-9).all())
+
+
+@pytest.mark.parametrize("lens, starts, G, H, kd, vd, dtype", [
+    ([256], [0], 1, 1, 1, 1, torch.float32), ([250, 3, 1, 9], [0, 7, 0, 2], 2, 4, 50, 33, torch.float32),
+    ([133, 300], [5, 0], 4, 8, 128, 256, torch.bfloat16), ([400], [1], 2, 2, 256, 300, torch.bfloat16),
+    ([2, 255], [3, 4], 3, 3, 257, 16, torch.float32)])
+def test_delta_prepare_of_many_rows(lens, starts, G, H, kd, vd, dtype):
+    """Runs of 8 rows that share their channels' inputs: sequences that begin and end inside a run, inputs from
+    the slots' histories, a sequence without a slot, key heads wider than the runs take."""
+    from types import SimpleNamespace
+    n = _native()
+    g = torch.Generator().manual_seed(kd)
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    R, B, taps = sum(lens), len(lens), 4
+    ch, mats = 2 * G * kd + H * vd, H * vd * kd
+    slots = [2 * b for b in range(B)]
+    if B > 2:
+        slots[1] = -1
+    row0 = [sum(lens[:b]) for b in range(B)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    ctx = SimpleNamespace(
+        row_pos=i32([s + i for s, m in zip(starts, lens) for i in range(m)]), n_seqs=B, seq_slot=i32(slots),
+        row_seq=i32([b for b, m in enumerate(lens) for _ in range(m)]), seq_start=i32(starts),
+        seq_end=i32([s + m for s, m in zip(starts, lens)]), seq_row0=i32(row0))
+    proj = rnd(R, ch + H * vd + 2 * H).to(dtype)
+    conv, a_log, bias = rnd(ch, taps), rnd(H), rnd(H)
+    state = rnd(2 * B, -(-(mats + (taps - 1) * ch) // 4) * 4)
+    outs = [torch.empty(R, m, device=DEV) for m in (G * kd, G * kd, H * vd, H, H)]
+    dev = state.clone().to(DEV)
+    n.delta_prepare(proj.to(DEV), conv.to(DEV), a_log.to(DEV), bias.to(DEV), dev, mats, *outs, ctx, H, G, kd, vd, taps)
+    q, k, v, beta, decay = (t.double().cpu() for t in outs)
+    x = proj.double()
+    for b in range(B):
+        rows = slice(row0[b], row0[b] + lens[b])
+        past = torch.zeros(taps - 1, ch, dtype=torch.float64)
+        if slots[b] >= 0:
+            past = state[slots[b], mats:mats + (taps - 1) * ch].double().view(taps - 1, ch)
+        full = torch.cat([past, x[rows, :ch]])
+        y = sum(full[j:j + lens[b]] * conv[:, j].double() for j in range(taps))
+        y = y * torch.sigmoid(y)
+        heads = y[:, :2 * G * kd].view(lens[b], 2 * G, kd)
+        size = torch.sqrt((heads * heads).sum(-1, keepdim=True) + 1e-6)
+        heads = heads / size
+        # (an activated sum is off by its terms' rounding, whatever it comes to; a unit norm divides that by
+        # the head's length, which is small where the sums cancel)
+        terms = sum(full[j:j + lens[b]].abs() * conv[:, j].double().abs() for j in range(taps))[:, :2 * G * kd]
+        off = 8 * 2.0 ** -24 * terms.view(lens[b], 2 * G, kd).amax(-1, keepdim=True) * kd ** 0.5 / size
+        want = (heads[:, :G].reshape(lens[b], -1) * kd ** -0.5, heads[:, G:].reshape(lens[b], -1), y[:, 2 * G * kd:],
+                torch.sigmoid(x[rows, ch + H * vd:ch + H * vd + H]),
+                torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(x[rows, ch + H * vd + H:] + bias.double())))
+        # (four products, an exponential and, for q and k, a sum of kd squares, a root and two divisions; the
+        # decay's exponent is of the size of ten)
+        for name, got, ref in zip("q k v beta decay".split(), (q, k, v, beta, decay), want):
+            room = (kd + 64) * 2.0 ** -24 * ref.abs().max()
+            if name in "qk":
+                room = room + (off[:, :G] * kd ** -0.5 if name == "q" else off[:, G:]).expand(-1, -1, kd).reshape(lens[b], -1)
+            assert bool(((got[rows] - ref).abs() <= room).all()), f"{name} of sequence {b}"
+        if slots[b] >= 0:
+            kept = dev[slots[b], mats:mats + (taps - 1) * ch].double().cpu().view(taps - 1, ch)
+            assert torch.equal(kept, full[lens[b]:])
