@@ -424,8 +424,13 @@ class Attention:
         # lengths do: 5 rows of 100 to 5 000 positions and one kv head take 12 us with blocks of 8
         # warps, 27 shared out.  Where a warp walks two tiles at most anyway there is nothing to share:
         # 8 rows of up to 1 088 seen positions, 8 kv heads of 128, take 10.6 us either way)
+        # Short windows and chunks stay with even runs as well: most rows are equally long under them, and
+        # the models that have them route rows to experts, where another order of sums decides
+        # near-ties of the choice anew (30 rows of 100 to 2 500 positions under a window of 1 024: sharing
+        # would save 3.6 % of the step).
         tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
-        if warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
+        unequal = self.chunk == 0 and (self.window == 0 or self.window >= 2048)
+        if unequal and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
             shared = shared_shape(R, self.nkv, tiles, self._resident_warps[4])
             if shared is not None:
                 slots, warps = shared
