@@ -1192,9 +1192,9 @@ def _scan_work(kind, rows, n_seqs, n_heads, key_dim, cols):
         7.0 * rows * n_heads * key_dim * cols
 
 
-# A step whose longest sequence has at least this many rows walks them in chunks (csrc/chunked_scan.cu)
-# instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us one by one and 83 in chunks, 300
-# rows 95 and 60 (4 heads of 64 x 64).
+# Where the caller allows it (``chunked``), a step whose longest sequence has at least this many rows walks
+# them in chunks (csrc/chunked_scan.cu) instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us
+# one by one and 83 in chunks, 300 rows 95 and 60 (4 heads of 64 x 64).
 CHUNKED_SCAN_MIN_ROWS = 160
 # ... unless the chunks' scratch memory would come to more 32-bit floats than this
 CHUNKED_SCAN_MAX_FLOATS = 1 << 29
@@ -1213,11 +1213,11 @@ def chunked_scan_scratch(out: torch.Tensor, ctx, n_heads: int, key_dim: int, col
     return torch.empty(n, dtype=torch.float32, device=out.device)
 
 
-@_timed(lambda qn, kn, vc, decay, beta, state, out, ctx, n_heads, n_kv, key_dim, value_dim: _scan_work(
+@_timed(lambda qn, kn, vc, decay, beta, state, out, ctx, n_heads, n_kv, key_dim, value_dim, chunked=True: _scan_work(
     "delta_scan", out.shape[0], ctx.n_seqs, n_heads, key_dim, value_dim))
 def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torch.Tensor,
                beta: torch.Tensor, state: torch.Tensor, out: torch.Tensor, ctx, n_heads: int,
-               n_kv: int, key_dim: int, value_dim: int) -> torch.Tensor:
+               n_kv: int, key_dim: int, value_dim: int, chunked: bool = True) -> torch.Tensor:
     """The gated delta rule over the step's rows, sequence by sequence, from and into the
     slots' matrices ``state[slot, :heads * value_dim * key_dim]``; ``out`` 32-bit
     ``[rows, heads * value_dim]``."""
@@ -1226,7 +1226,7 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torc
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("delta_scan: the state is too small for the matrices")
-    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim, delta=True)
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim, delta=True) if chunked else None
     if scratch is not None:
         _check(library().sib_delta_scan_chunked(
             _ptr(qn), _ptr(kn), _ptr(vc), _ptr(decay), _ptr(beta), _ptr(state),
@@ -1242,11 +1242,11 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torc
     return out
 
 
-@_timed(lambda proj, bias_i, bias_f, cap, state, out, m_out, ctx, n_heads, key_dim, value_dim: _scan_work(
+@_timed(lambda proj, bias_i, bias_f, cap, state, out, m_out, ctx, n_heads, key_dim, value_dim, chunked=True: _scan_work(
     "memory_scan", out.shape[0], ctx.n_seqs, n_heads, key_dim, value_dim + 1))
 def memory_scan(proj: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
                 state: torch.Tensor, out: torch.Tensor, m_out: torch.Tensor, ctx, n_heads: int,
-                key_dim: int, value_dim: int) -> torch.Tensor:
+                key_dim: int, value_dim: int, chunked: bool = True) -> torch.Tensor:
     """The matrix memory with exponential gates over the step's rows.  ``proj``:
     ``[q | k | v | gate | i | f]`` per row; ``out`` 32-bit ``[rows, heads * (value_dim + 1)]``
     (the last column of a head is <n, q>), ``m_out`` ``[rows, heads]`` the running maxima;
@@ -1263,7 +1263,7 @@ def memory_scan(proj: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, 
     _f32(m_out, rows * n_heads, "m_out")
     if state.shape[1] < n_heads * (value_dim + 1) * key_dim + n_heads:
         raise KernelError("memory_scan: the state is too small")
-    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim + 1, memory=True)
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim + 1, memory=True) if chunked else None
     if scratch is not None:
         _check(library().sib_memory_scan_chunked(
             _ptr(proj), c_longlong(proj.stride(0)), _code(proj.dtype), c_longlong(2 * nq + 2 * nv),
@@ -1305,11 +1305,11 @@ def retention_prepare(proj: torch.Tensor, inv_freq: Optional[torch.Tensor], rot:
         c_int(key_dim), c_int(value_dim), c_float(k_scale), c_int(1 if silu else 0), _stream()))
 
 
-@_timed(lambda qn, kn, vc, decay, state, out, ctx, n_heads, key_dim, value_dim: _scan_work(
+@_timed(lambda qn, kn, vc, decay, state, out, ctx, n_heads, key_dim, value_dim, chunked=True: _scan_work(
     "retention_scan", out.shape[0], ctx.n_seqs, n_heads, key_dim, value_dim))
 def retention_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: torch.Tensor,
                    state: torch.Tensor, out: torch.Tensor, ctx, n_heads: int, key_dim: int,
-                   value_dim: int) -> torch.Tensor:
+                   value_dim: int, chunked: bool = True) -> torch.Tensor:
     """S <- decay_h S + k v^T, o = S^T q over the step's rows, sequence by sequence, from and
     into the slots' matrices ``state[slot, :heads * value_dim * key_dim]``; ``out`` 32-bit
     ``[rows, heads * value_dim]``; ``decay`` one 32-bit value per head."""
@@ -1322,7 +1322,7 @@ def retention_scan(qn: torch.Tensor, kn: torch.Tensor, vc: torch.Tensor, decay: 
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("retention_scan: the state is too small for the matrices")
-    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim)
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim) if chunked else None
     if scratch is not None:
         nq, nv = n_heads * key_dim, n_heads * value_dim
         _check(library().sib_gated_scan_chunked(
@@ -1370,11 +1370,11 @@ def head_norm_gate(o: torch.Tensor, m: Optional[torch.Tensor], w: Optional[torch
     return y
 
 
-@_timed(lambda q, k, v, keep, take, state, out, ctx, n_heads, n_kv, key_dim, value_dim: _scan_work(
+@_timed(lambda q, k, v, keep, take, state, out, ctx, n_heads, n_kv, key_dim, value_dim, chunked=True: _scan_work(
     "gated_scan", out.shape[0], ctx.n_seqs, n_heads, key_dim, value_dim))
 def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, keep: torch.Tensor,
                take: torch.Tensor, state: torch.Tensor, out: torch.Tensor, ctx, n_heads: int,
-               n_kv: int, key_dim: int, value_dim: int) -> torch.Tensor:
+               n_kv: int, key_dim: int, value_dim: int, chunked: bool = True) -> torch.Tensor:
     """S <- keep S + take k v^T, o = S^T q with ``keep`` and ``take`` 32-bit ``[rows, heads]``
     (csrc/recurrent.cu).  ``q``, ``k`` (``n_kv`` key heads of ``key_dim``) and ``v`` (``n_heads``
     heads of ``value_dim``) are 32-bit views whose rows may be columns of one buffer."""
@@ -1389,7 +1389,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, keep: torch.Te
     _f32(out, rows * n_heads * value_dim, "out")
     if state.shape[1] < n_heads * value_dim * key_dim:
         raise KernelError("gated_scan: the state is too small for the matrices")
-    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim)
+    scratch = chunked_scan_scratch(out, ctx, n_heads, key_dim, value_dim) if chunked else None
     if scratch is not None:
         _check(library().sib_gated_scan_chunked(
             _ptr(q), _ptr(k), _ptr(v), c_longlong(q.stride(0)), c_longlong(k.stride(0)),

@@ -115,6 +115,12 @@ class Runtime:
         # SIB_EARLY_KEYS=0: the attention over the cache fetches no keys before the kernel ahead
         # of it has finished
         self.early_keys = os.environ.get("SIB_EARLY_KEYS", "1") != "0"
+        # True: the recurrences of long prompts go in chunks of 64 tokens (csrc/chunked_scan.cu): 2 048 rows of 8
+        # heads of 128 x 256 in 255 us (delta rule) and 163 (gated) instead of 702 and 639, but the outputs are
+        # 1.3e-7 to 1.7e-7 off against 64 bits instead of 0.9e-7, and each call takes scratch memory.  So it is off
+        # unless an engine's owner sets it before the first step: a matrix memory divides by sums that nearly
+        # cancel, and the logits of a bfloat16 model of 8 layers differ by 2 to 3 % between the two.
+        self.chunked_scans = False
         # SIB_DECODE_CHAIN=1: the steps between two attention kernels of a step of few rows run
         # as ONE chain kernel (csrc/decode_chain.cu) instead of one kernel each.  Measured on
         # the Gemma2-2B shape it is the slower of the two so far (a layer's products and norms:

@@ -166,7 +166,7 @@ class GatedDeltaRule:
         native.delta_prepare(proj, self.conv_w, self.a_log, self.dt_bias, state, self.matrices,
                              qn, kn, vc, beta, decay, ctx, H, G, kd, vd, self.taps)
         o = torch.empty((R, H * vd), **f32)
-        native.delta_scan(qn, kn, vc, decay, beta, state, o, ctx, H, G, kd, vd)
+        native.delta_scan(qn, kn, vc, decay, beta, state, o, ctx, H, G, kd, vd, chunked=rt.chunked_scans)
         y = torch.empty((R, H * vd), dtype=proj.dtype, device=x.device)
         gate = proj[:, self.channels:self.channels + H * vd]
         native.head_norm_gate(o, None, self.norm_gain, gate, y, H, vd, self.eps, native.GATE_SILU)
@@ -239,7 +239,8 @@ class MatrixMemory:
         proj = rt.linear(x, self.w_in)
         o = torch.empty((R, H * (vd + 1)), dtype=torch.float32, device=x.device)
         m = torch.empty((R, H), dtype=torch.float32, device=x.device)
-        native.memory_scan(proj, self.bias_i, self.bias_f, self.cap, state, o, m, ctx, H, kd, vd)
+        native.memory_scan(proj, self.bias_i, self.bias_f, self.cap, state, o, m, ctx, H, kd, vd,
+                           chunked=rt.chunked_scans)
         y = torch.empty((R, H * vd), dtype=proj.dtype, device=x.device)
         gate = proj[:, 2 * H * kd + H * vd:2 * H * kd + 2 * H * vd]
         native.head_norm_gate(o, m, self.norm_gain, gate, y, H, vd, self.eps, native.GATE_SIGMOID)
@@ -328,7 +329,7 @@ class Retention:
         native.retention_prepare(proj, self.inv_freq, self.rot, ctx.row_pos, qn, kn, vc, H, kd, vd,
                                  self.key_scale, self.silu_inputs)
         o = torch.empty((R, H * vd), **f32)
-        native.retention_scan(qn, kn, vc, self.decay, state, o, ctx, H, kd, vd)
+        native.retention_scan(qn, kn, vc, self.decay, state, o, ctx, H, kd, vd, chunked=rt.chunked_scans)
         y = torch.empty((R, H * vd), dtype=proj.dtype, device=x.device)
         gate = proj[:, 2 * H * kd + H * vd:2 * H * kd + 2 * H * vd]
         # (one root mean square over all heads: the row as a single head of heads * vd columns)
@@ -417,7 +418,7 @@ class StateSpace:
                            self.matrices, xbc, keep, take, ctx, H, self.inner, self.channels, self.taps)
         o = torch.empty((R, self.inner), **f32)
         native.gated_scan(xbc[:, self.inner + G * N:], xbc[:, self.inner:self.inner + G * N],
-                          xbc[:, :self.inner], keep, take, state, o, ctx, H, G, N, P)
+                          xbc[:, :self.inner], keep, take, state, o, ctx, H, G, N, P, chunked=rt.chunked_scans)
         y = torch.empty((R, self.inner), dtype=proj.dtype, device=x.device)
         native.ssm_finish(o, xbc, proj[:, :self.inner], self.skip, self.norm_gain, y, self.inner, P,
                           self.parts, self.eps)
