@@ -226,8 +226,10 @@ __global__ void __launch_bounds__(128) delta_prepare_runs_kernel(DeltaPrepareArg
     }
     channels8(unit * p.kd, (unit + 1) * p.kd, [&](int r, const float (&y)[8]) {
         float ss = 0.f;
+        // (channels beyond kd gave silu(0) = 0.  Product and sum are rounded one after the other, as the sum over
+        // two rounds of 256 channels above comes to: a row's q and k are the same bits in either form)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss += y[i] * y[i];       // (channels beyond kd gave silu(0) = 0)
+        for (int i = 0; i < 8; ++i) ss = __fadd_rn(ss, __fmul_rn(y[i], y[i]));
         float inv = 1.0f / sqrtf(warp_sum(ss) + 1e-6f);
         if (unit < p.G) inv *= 1.0f / sqrtf((float)p.kd);
         float* dst = (unit < p.G ? p.qn : p.kn) + (size_t)r * nqk + (size_t)(unit % p.G) * p.kd;

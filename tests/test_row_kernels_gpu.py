@@ -132,3 +132,34 @@ def test_delta_prepare_of_many_rows(lens, starts, G, H, kd, vd, dtype):
         if slots[b] >= 0:
             kept = dev[slots[b], mats:mats + (taps - 1) * ch].double().cpu().view(taps - 1, ch)
             assert torch.equal(kept, full[lens[b]:])
+
+
+def test_delta_prepare_does_not_depend_on_what_is_beside_a_sequence():
+    """Runs of 8 rows give the same bits as rows one by one: ten sequences in one call against each alone."""
+    from types import SimpleNamespace
+    n = _native()
+    g = torch.Generator().manual_seed(12)
+    G, H, kd, vd, taps, lens = 2, 4, 100, 72, 4, [205 + 3 * b for b in range(10)]
+    ch, mats = 2 * G * kd + H * vd, 16
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    proj = torch.randn(sum(lens), ch + H * vd + 2 * H, generator=g).to(torch.bfloat16).to(DEV)
+    conv, a_log, bias = (torch.randn(*s, generator=g).to(DEV) for s in ((ch, taps), (H,), (H,)))
+    first = torch.randn(10, mats + (taps - 1) * ch, generator=g).to(DEV)
+
+    def prepare(seqs, rows, state):
+        m = [lens[b] for b in seqs]
+        ctx = SimpleNamespace(
+            row_pos=i32([9 + i for k in m for i in range(k)]), n_seqs=len(m), seq_slot=i32(seqs),
+            row_seq=i32([b for b, k in enumerate(m) for _ in range(k)]), seq_start=i32([9] * len(m)),
+            seq_end=i32([9 + k for k in m]), seq_row0=i32([sum(m[:b]) for b in range(len(m))]))
+        outs = [torch.empty(sum(m), w, device=DEV) for w in (G * kd, G * kd, H * vd, H, H)]
+        n.delta_prepare(proj[rows], conv, a_log, bias, state, mats, *outs, ctx, H, G, kd, vd, taps)
+        return outs
+
+    together, alone = first.clone(), first.clone()
+    got, at = prepare(list(range(10)), slice(0, sum(lens)), together), 0
+    for b, k in enumerate(lens):
+        for name, x, y in zip("q k v beta decay".split(), got, prepare([b], slice(at, at + k), alone)):
+            assert torch.equal(x[at:at + k], y), f"{name} of sequence {b}"
+        at += k
+    assert torch.equal(together, alone)
