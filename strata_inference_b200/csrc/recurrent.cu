@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(DeltaPrepareArgs p) 
 
 // The same for many rows, 4 taps and kd <= 256: a warp takes a unit of RUN consecutive rows, keeps its channels'
 // taps in registers and moves their last inputs along, so that a row costs one load a channel instead
-// of four and four of weights (2 048 rows of 4 + 4 heads of 128 and 8 of 256: 57.6 -> 36.6 us).
+// of four and four of weights (2 048 rows of 4 + 4 heads of 128 and 8 of 256: 79 -> 60 us, 59 -> 37 with the rows
+// still in L2).
 constexpr int kRunRows = 8;
 template <typename T>
 __global__ void __launch_bounds__(128) delta_prepare_runs_kernel(DeltaPrepareArgs p, int rows) {
@@ -593,6 +594,16 @@ static int check_scan(const char* what, int rows, int n_seqs, int H, int G, int 
     return 0;
 }
 
+// Whether the inputs of a step of `rows` rows in `n_seqs` sequences are made in runs of 8 rows.  A run's rows come one
+// after the other, an eighth of the warps for a chain eight times as long, so it takes about 24 000 (row, unit) pairs
+// to fill the device with them (4 + 4 + 8 heads of 128 and 256, one prompt, rows cold in L2, rows one by one -> in runs:
+// 256 rows 22 -> 36 us, 1 024 rows 46 -> 40, 1 536 rows 63 -> 58, 4 096 rows 144 -> 105; 2 + 2 + 4 heads of 64: 1 536
+// rows 26 -> 30, 4 096 rows 56 -> 48), and neighbours to share with: a sequence's first row in a run loads its
+// history (256 sequences of one token 24 -> 46 us, 2 048 of one 113 -> 118, 512 of four 87 -> 62).
+SIB_EXPORT int sib_delta_prepare_in_runs(int rows, int n_seqs, int H, int G, int kd, int taps) {
+    return taps == 4 && kd <= 256 && rows >= 4ll * n_seqs && (long long)rows * (2 * G + H + 1) >= 24000;
+}
+
 SIB_EXPORT int sib_delta_prepare(
     const void* proj, long long stride, int dtype, const float* conv_w, const float* a_log,
     const float* dt_bias, float* state, long long state_stride, long long hist_offset, float* qn,
@@ -609,8 +620,7 @@ SIB_EXPORT int sib_delta_prepare(
                        row_seq, seq_slot, seq_start, seq_row0, stride, state_stride, hist_offset,
                        H, G, kd, vd, taps};
     cudaStream_t s = (cudaStream_t)stream;
-    // (single-token steps have no neighbours to share with; from 256 rows on the runs' warps fill the device)
-    if (taps == 4 && kd <= 256 && rows >= 256 && ((uintptr_t)conv_w % 16) == 0)
+    if (sib_delta_prepare_in_runs(rows, n_seqs, H, G, kd, taps) && ((uintptr_t)conv_w % 16) == 0)
         SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(delta_prepare_runs_kernel<T>,
                                                      dim3((rows + kRunRows - 1) / kRunRows, (units + 3) / 4), dim3(128), 0,
                                                      s, p, rows));

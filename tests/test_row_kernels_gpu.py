@@ -77,7 +77,10 @@ def test_head_norm_gate(rows, heads, vd, memory, act):
 @pytest.mark.parametrize("lens, starts, G, H, kd, vd, dtype", [
     ([256], [0], 1, 1, 1, 1, torch.float32), ([250, 3, 1, 9], [0, 7, 0, 2], 2, 4, 50, 33, torch.float32),
     ([133, 300], [5, 0], 4, 8, 128, 256, torch.bfloat16), ([400], [1], 2, 2, 256, 300, torch.bfloat16),
-    ([2, 255], [3, 4], 3, 3, 257, 16, torch.float32)])
+    ([2, 255], [3, 4], 3, 3, 257, 16, torch.float32),
+    # (enough rows and heads for the runs)
+    ([24000], [0], 1, 1, 1, 1, torch.float32), ([690, 3, 1, 34], [0, 7, 0, 2], 8, 16, 50, 33, torch.float32),
+    ([1133, 300], [5, 0], 4, 8, 128, 256, torch.bfloat16), ([1001], [1], 8, 8, 256, 300, torch.bfloat16)])
 def test_delta_prepare_of_many_rows(lens, starts, G, H, kd, vd, dtype):
     """Runs of 8 rows that share their channels' inputs: sequences that begin and end inside a run, inputs from
     the slots' histories, a sequence without a slot, key heads wider than the runs take."""
@@ -139,7 +142,7 @@ def test_delta_prepare_does_not_depend_on_what_is_beside_a_sequence():
     from types import SimpleNamespace
     n = _native()
     g = torch.Generator().manual_seed(12)
-    G, H, kd, vd, taps, lens = 2, 4, 100, 72, 4, [205 + 3 * b for b in range(10)]
+    G, H, kd, vd, taps, lens = 4, 8, 100, 72, 4, [205 + 3 * b for b in range(10)]
     ch, mats = 2 * G * kd + H * vd, 16
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
     proj = torch.randn(sum(lens), ch + H * vd + 2 * H, generator=g).to(torch.bfloat16).to(DEV)
