@@ -420,17 +420,22 @@ class Attention:
         rows' lengths where ``shared_shape`` has a shape for it, else as many for every row."""
         rt, R = self.rt, ctx.n_rows
         runs, warps = self._decode_shape(ctx, ctx.cache.max_seq_len)
-        # (few (row, kv head) pairs have many runs each, and joining those costs more than unequal
+        # Few (row, kv head) pairs have many runs each, and joining those costs more than unequal
         # lengths do: 5 rows of 100 to 5 000 positions and one kv head take 12 us with blocks of 8
         # warps, 27 shared out.  Where a warp walks two tiles at most anyway there is nothing to share:
-        # 8 rows of up to 1 088 seen positions, 8 kv heads of 128, take 10.6 us either way)
-        # Short windows and chunks stay with even runs as well: most rows are equally long under them, and
-        # the models that have them route rows to experts, where another order of sums decides
-        # near-ties of the choice anew (30 rows of 100 to 2 500 positions under a window of 1 024: sharing
-        # would save 3.6 % of the step).
+        # 8 rows of up to 1 088 seen positions, 8 kv heads of 128, take 10.6 us either way.
+        # Under a short window most rows are equally long, and then sharing is the slower of the two (32 heads on
+        # 8 kv heads of 128, window 1 024, even -> shared out: 32 rows of 4 000 positions 45 -> 51 us, 64 rows 78 ->
+        # 86, where rows of 100 to 3 000 positions gain 43 -> 39 and 72 -> 64); from a window of 2 048 on equal rows
+        # lose 0 to 3 % (8 heads on 4 kv heads of 256: 8 rows 24.6 -> 24.8, 64 rows 95 -> 96) and unequal ones gain up to
+        # 45 %.  Rows lie anywhere in their chunks (16 heads on 8 kv heads of 128, 32 rows at random positions: chunks
+        # of 512 21 -> 19 us, of 2 048 50 -> 35).
+        # A model with parts that make much of a last bit keeps even runs (Runtime.steady_sums): shared out, the order
+        # of a row's sums would depend on the other rows' lengths (decode steps of a Karupel of 8 layers: logits
+        # up to 3 % apart; what that costs: 32 rows of 150 to 3 001 positions, 16 heads on 8 kv heads of 128, 64 us instead of 35).
         tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
-        unequal = self.chunk == 0 and (self.window == 0 or self.window >= 2048)
-        if unequal and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
+        shares = not rt.steady_sums and (self.window == 0 or self.window >= 2048)
+        if shares and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
             shared = shared_shape(R, self.nkv, tiles, self._resident_warps[4])
             if shared is not None:
                 slots, warps = shared

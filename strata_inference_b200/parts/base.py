@@ -115,6 +115,11 @@ class Runtime:
         # SIB_EARLY_KEYS=0: the attention over the cache fetches no keys before the kernel ahead
         # of it has finished
         self.early_keys = os.environ.get("SIB_EARLY_KEYS", "1") != "0"
+        # Set by parts in which a last bit of their inputs can come to much (routed experts choose by near-ties, a
+        # recurrence divides by sums that nearly cancel and carries the rest along): the attention over the cache
+        # then cuts a row's keys into even runs, whatever else is in the step, and leaves its blocks to no rule
+        # that would order the sums by the other rows' lengths (parts/attention.py _decode_launch).
+        self.steady_sums = False
         # True: the recurrences of long prompts go in chunks of 64 tokens (csrc/chunked_scan.cu): 2 048 rows of 8
         # heads of 128 x 256 in 255 us (delta rule) and 163 (gated) instead of 702 and 639, but the outputs are
         # 1.3e-7 to 1.7e-7 off against 64 bits instead of 0.9e-7, and each call takes scratch memory.  So it is off

@@ -327,6 +327,7 @@ class RoutedExperts:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (a last bit decides near-ties of the choice)
         self.hidden = hidden
         self.E, self.top, self.ff, self.sff = self._sizes(params)
         self.form = self._form(params)

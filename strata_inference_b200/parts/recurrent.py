@@ -137,6 +137,7 @@ class GatedDeltaRule:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (what the state and its divisors make of a last bit)
         self.H, self.G, self.kd, self.vd, self.taps = self._sizes(params)
         self.eps = float(params["norm_eps"])
         self.channels = 2 * self.G * self.kd + self.H * self.vd
@@ -215,6 +216,7 @@ class MatrixMemory:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (what the state and its divisors make of a last bit)
         self.H, self.kd, self.vd = self._sizes(params)
         self.eps = float(params["norm_eps"])
         self.cap = float(params["gate_cap"])
@@ -286,6 +288,7 @@ class Retention:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (what the state and its divisors make of a last bit)
         self.H, self.kd, self.vd = self._sizes(params)
         self.eps = float(params["norm_eps"])
         self.key_scale = float(params.get("key_scale", 1.0))
@@ -388,6 +391,7 @@ class StateSpace:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (what the state and its divisors make of a last bit)
         self.H, self.P, self.N, self.G, self.taps, self.parts = self._sizes(params)
         self.eps = float(params["norm_eps"])
         self.inner = self.H * self.P
@@ -472,6 +476,7 @@ class GeneralDelta:
 
     def __init__(self, params: Mapping, hidden: int, weights: Mapping[str, torch.Tensor], rt):
         self.rt = rt
+        rt.steady_sums = True        # (what the state and its divisors make of a last bit)
         self.H, self.d, self.rank = self._sizes(params)
         self.eps = float(params["norm_eps"])
         self.w_in = rt.cast_matrix(weights["in_proj.weight"])
