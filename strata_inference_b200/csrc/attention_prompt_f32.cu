@@ -126,35 +126,50 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prompt_f32_kernel(Prompt
         // ---- scores: this warp's dimensions of all 32 x 32 ----
         {
             const int rg = lane >> 3, kg = lane & 7;      // pairs rg + 4 i, keys kg + 8 j
-            float s[8][4];
+            // (the even and the odd dimensions of 16 as two sums, then the sums' sum: as a single sum of 64 products
+            // scores were further from 64 bits than the general kernel's, which adds 8 a lane and then by pairs)
+            float sum[8][4];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+                for (int j = 0; j < 4; ++j) sum[i][j] = 0.f;
             const float* qb = Qs + rg * KS + warp * DW;
             const float* kb = Ks + kg * KS + warp * DW;
-#pragma unroll 2
-            for (int d = 0; d < DW; d += 4) {
-                float4 q[8], k[4];
+#pragma unroll 1
+            for (int d0 = 0; d0 < DW; d0 += 16) {
+                uint64_t s[8][4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(kb + 8 * j * KS + d);
+                for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const float4*>(qb + 4 * i * KS + d);
+                    for (int j = 0; j < 4; ++j) s[i][j] = 0ull;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int d = d0; d < d0 + 16; d += 4) {
+                    ulonglong2 q[8], k[4];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        s[i][j] += q[i].x * k[j].x;
-                        s[i][j] += q[i].y * k[j].y;
-                        s[i][j] += q[i].z * k[j].z;
-                        s[i][j] += q[i].w * k[j].w;
+                    for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(kb + 8 * j * KS + d);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const ulonglong2*>(qb + 4 * i * KS + d);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            fma2(s[i][j], q[i].x, k[j].x);
+                            fma2(s[i][j], q[i].y, k[j].y);
+                        }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 x = unpair(s[i][j]);
+                        sum[i][j] += x.x + x.y;
                     }
             }
             float* part = Sp + warp * PAIRS * SS;
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[(rg + 4 * i) * SS + kg + 8 * j] = s[i][j];
+                for (int j = 0; j < 4; ++j) part[(rg + 4 * i) * SS + kg + 8 * j] = sum[i][j];
         }
         __syncthreads();                                  // the parts are there; K is free
         copy_rows(p.v, t);
