@@ -1638,8 +1638,10 @@ def attention_decode_resident_warps(n_heads: int, n_kv: int, head_dim: int, warp
                                                                 c_int(head_dim), c_int(warps)))
 
 
-# 32-bit prompts whose longest has at least this many rows go to the tiled kernel
-ATTENTION_PROMPT_F32_MIN_ROWS = 2
+# 32-bit prompts whose longest has at least this many rows go to the tiled kernel (16 prompts, 8 heads of 256,
+# tiled against the general kernel: of 2 rows 16 and 10 us, of 5 rows 16 and 12, of 16 rows 18 and 21, of 32
+# rows 18 and 43)
+ATTENTION_PROMPT_F32_MIN_ROWS = 16
 
 
 def attention_prompt_f32_supports(n_heads: int, n_kv: int, head_dim: int) -> bool:

@@ -106,3 +106,16 @@ def test_no_further_from_64_bits_than_the_general_kernel(lens, nh, nkv, hd, cap,
     want = torch.cat([_plain(qkv[r:r + n], nh, nkv, hd, scale, cap, 0, 0, 0, None) for r, n in zip(row0, lens)])
     off = [(y.double() - want).norm().item() for y in (tiled, out.cpu())]
     assert off[0] <= 1.05 * off[1], f"{off[0] / off[1]:.3f} of the general kernel's error"
+
+
+@pytest.mark.parametrize("lengths,tiled", [([3, 8], False), ([2, 16], True)])
+def test_the_shortest_prompts_stay_with_the_general_kernel(lengths, tiled, monkeypatch):
+    from helpers import TINY_A
+    from strata_inference_b200 import Engine
+    from strata_inference_b200.kernels import native
+    native.library()
+    calls, plain = [], native.attention_prompt_f32
+    monkeypatch.setattr(native, "attention_prompt_f32", lambda *a, **kw: (calls.append(1), plain(*a, **kw))[1])
+    eng = Engine.from_random(TINY_A, 1, dtype="float32", max_tokens=256)
+    eng.step([(eng.new_sequence(), [5 + i for i in range(n)]) for n in lengths])
+    assert bool(calls) == tiled
