@@ -3,17 +3,19 @@
 // kept first positions, sink, softmax, weighted sum), in tiles.
 //
 // attention_rows.cu gives every (row, head) a warp that reads every key and value it sees by itself:
-// two prompts of 301 and 700 rows, 8 heads of 256 on 4 kv heads, took 684 us, 3.5 TFLOP/s, waiting for L2.
-// Here a block takes 32 (row, query head) pairs of one kv head and walks the keys 64 at a time:
+// two prompts of 301 and 700 rows, 8 heads of 256 on 4 kv heads, took 711 us, 3.5 TFLOP/s, waiting for L2 (here: 162).
+// Here a block of four warps takes 32 (row, query head) pairs of one kv head and walks the keys 32 at a time:
 //
-// * scores: 8 pairs x 8 keys a thread, a word of shared memory for 4 FMAs (what the 128 bytes a cycle
-//   of shared memory feed the FMA units with).  One warp covers the 32 x 64 scores, so the four warps
-//   take a quarter of the head's dimensions each and their parts are added by the softmax;
+// * scores: 8 pairs x 4 keys a thread, 12 words of shared memory for 32 FMAs.  One warp covers the 32 x 32 scores, so the
+//   four warps take a quarter of the head's dimensions each and their parts are added by the softmax;
 // * weighted sum: 8 pairs a warp, every lane its own columns, the weights read by the whole warp at once;
-// * K of the next tile is copied (cp.async) during the weighted sum, V of this one during the scores.
+// * K and V share one buffer, so that two blocks fit an SM at 256 dimensions: V is copied (cp.async) during
+//   the softmax, K of the next tile once the weighted sum is done with V.  Neither copy hides behind its own
+//   block's products; the other resident block's do that.
 //
-// The longest blocks start first.  FMAs bound it: 1.2 G of them for the prompts above, 33 us at the rate of
-// all SMs.  A key that a row may not see is left out of its sum, not multiplied by zero.
+// The longest blocks start first.  FMAs would bound it: 1.2 G of them for the prompts above, 33 us at the rate of
+// all SMs; with two warps a scheduler it is the latencies of shared memory and of the exposed copies.  A key
+// that a row may not see is left out of its sum, not multiplied by zero.
 //
 // Plain counterpart: tests/plain_gemma2.py attention().
 #include "common.cuh"
