@@ -1192,19 +1192,23 @@ def _scan_work(kind, rows, n_seqs, n_heads, key_dim, cols):
         7.0 * rows * n_heads * key_dim * cols
 
 
-# Where the caller allows it (``chunked``), a step whose longest sequence has at least this many rows walks
-# them in chunks (csrc/chunked_scan.cu) instead of one by one: 8 heads of 128 x 256, delta rule, 128 rows 56 us
-# one by one and 83 in chunks, 300 rows 95 and 60 (4 heads of 64 x 64).
-CHUNKED_SCAN_MIN_ROWS = 160
-# ... unless the chunks' scratch memory would come to more 32-bit floats than this
+# Where the caller allows it (``chunked``), a step walks its sequences in chunks (csrc/chunked_scan.cu) instead of row
+# by row if the longest has at least this many rows, and if there are a quarter as many rows for every sequence: a chunk
+# costs the same whether it holds 64 rows or one, and a sequence row by row next to nothing.  8 heads of 128 x 256,
+# delta rule and gated, row by row -> in chunks: one sequence of 160 rows 63 -> 87 and 58 -> 56 us, of 300 rows 111 ->
+# 93 and 101 -> 60, of 2 048 rows 702 -> 255 and 639 -> 163; eight of 300 rows 341 -> 325 and 309 -> 214; one of
+# 300 beside 7 single tokens 129 -> 156 and 114 -> 126, one of 2 048 beside 30 of them 819 -> 458 and 724 -> 400,
+# beside 60 (not taken) 827 -> 685 and 736 -> 689, beside 200 846 -> 1 689 and 752 -> 1 885.
+CHUNKED_SCAN_MIN_ROWS = 256
+# ... unless the chunks' scratch memory would come to more 32-bit floats than this, or cannot be had
 CHUNKED_SCAN_MAX_FLOATS = 1 << 29
 
 
 def chunked_scan_scratch(out: torch.Tensor, ctx, n_heads: int, key_dim: int, cols: int, delta: bool = False,
                          memory: bool = False) -> Optional[torch.Tensor]:
-    """Scratch memory of a scan in chunks; None where the scan goes row by row: no sequence of the
-    step is long enough, the kernel does not take the key width, or it would need too much."""
-    if ctx.max_count < CHUNKED_SCAN_MIN_ROWS:
+    """Scratch memory of a scan in chunks; None where the scan goes row by row: the step's sequences are
+    not long enough, the kernel does not take the key width, or it would need too much."""
+    if ctx.max_count < CHUNKED_SCAN_MIN_ROWS or out.shape[0] < CHUNKED_SCAN_MIN_ROWS // 4 * ctx.n_seqs:
         return None
     n = library().sib_chunked_scan_floats(c_longlong(out.shape[0]), c_int(ctx.n_seqs), c_int(n_heads), c_int(key_dim),
                                           c_int(cols), c_int(1 if delta else 0), c_int(1 if memory else 0))

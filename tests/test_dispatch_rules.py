@@ -1,6 +1,9 @@
 """Which form of a kernel a call takes: the rules that the library answers without a device."""
 
 from ctypes import c_int
+from types import SimpleNamespace
+
+import torch
 
 from strata_inference_b200.kernels import native
 
@@ -15,3 +18,15 @@ def test_delta_prepare_takes_runs_where_sequences_are_long_and_rows_are_many():
         assert not any(_in_runs(rows, 1, *heads) for rows in (1, 8, 256, 500)), "short prompts"
         assert all(_in_runs(rows, n, *heads) for rows, n in ((4096, 1), (4096, 1024), (8192, 61)))
     assert not _in_runs(4096, 1, 8, 4, kd=257) and not _in_runs(4096, 1, 8, 4, taps=3)
+
+
+def _chunks(lens, H=8, kd=128, cols=256):
+    ctx = SimpleNamespace(max_count=max(lens), n_seqs=len(lens))
+    return native.chunked_scan_scratch(torch.empty(sum(lens), 1), ctx, H, kd, cols, delta=True) is not None
+
+
+def test_scans_go_in_chunks_where_most_rows_are_in_long_sequences():
+    assert _chunks([300]) and _chunks([2048]) and _chunks([300] * 8) and _chunks([2048] + [1] * 30)
+    assert not _chunks([255]) and not _chunks([100] * 40)
+    assert not _chunks([300] + [1] * 7) and not _chunks([160] + [1] * 60) and not _chunks([2048] + [1] * 200)
+    assert not _chunks([2048], kd=129) and not _chunks([4096] * 16, H=32)
