@@ -1206,15 +1206,18 @@ CHUNKED_SCAN_MAX_FLOATS = 1 << 29
 
 def chunked_scan_scratch(out: torch.Tensor, ctx, n_heads: int, key_dim: int, cols: int, delta: bool = False,
                          memory: bool = False) -> Optional[torch.Tensor]:
-    """Scratch memory of a scan in chunks; None where the scan goes row by row: the step's sequences are
-    not long enough, the kernel does not take the key width, or it would need too much."""
+    """Scratch memory of a scan in chunks; None where the scan goes row by row, which needs none: the step's
+    sequences are not long enough, the kernel does not take the key width, or it would need too much."""
     if ctx.max_count < CHUNKED_SCAN_MIN_ROWS or out.shape[0] < CHUNKED_SCAN_MIN_ROWS // 4 * ctx.n_seqs:
         return None
     n = library().sib_chunked_scan_floats(c_longlong(out.shape[0]), c_int(ctx.n_seqs), c_int(n_heads), c_int(key_dim),
                                           c_int(cols), c_int(1 if delta else 0), c_int(1 if memory else 0))
     if not 0 < n <= CHUNKED_SCAN_MAX_FLOATS:
         return None
-    return torch.empty(n, dtype=torch.float32, device=out.device)
+    try:
+        return torch.empty(n, dtype=torch.float32, device=out.device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 @_timed(lambda qn, kn, vc, decay, beta, state, out, ctx, n_heads, n_kv, key_dim, value_dim, chunked=True: _scan_work(

@@ -30,3 +30,13 @@ def test_scans_go_in_chunks_where_most_rows_are_in_long_sequences():
     assert not _chunks([255]) and not _chunks([100] * 40)
     assert not _chunks([300] + [1] * 7) and not _chunks([160] + [1] * 60) and not _chunks([2048] + [1] * 200)
     assert not _chunks([2048], kd=129) and not _chunks([4096] * 16, H=32)
+
+
+def test_a_scan_goes_row_by_row_where_the_memory_of_its_chunks_cannot_be_had(monkeypatch):
+    def empty(*a, **kw):
+        raise torch.OutOfMemoryError("no memory is left")
+
+    ctx, out = SimpleNamespace(max_count=2048, n_seqs=1), torch.empty(2048, 1)
+    assert native.chunked_scan_scratch(out, ctx, 8, 128, 256) is not None
+    monkeypatch.setattr(native.torch, "empty", empty)
+    assert native.chunked_scan_scratch(out, ctx, 8, 128, 256) is None
