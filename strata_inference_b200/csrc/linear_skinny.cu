@@ -146,15 +146,15 @@ __device__ __forceinline__ void skinny_linear_body(
     const uint4 zero = make_uint4(0, 0, 0, 0);
 
     // The weights do not depend on the kernel before this one: pull this block's towards L2 while
-    // that kernel is still running, then wait for it.  Where there are more blocks than the device
-    // holds, a block asks for its runs of 8 rows, which are contiguous, as a whole, and for those of the
+    // that kernel is still running, then wait for it.  In grids that sib_skinny_linear_ahead names, a
+    // block asks for its runs of 8 rows, which are contiguous, as a whole, and for those of the
     // block that takes its place on the SM: else the memory idles between the first blocks' last
     // loads and the next ones' first.  (Gemma2-2B shape, batch 1: gate/up product, 1 152 blocks of which
-    // 592 are resident, 16.5 -> 14.4 us, logits 188 -> 177 us.)  Blocks that are all resident ask line by
+    // 592 are resident, 16.5 -> 14.4 us, logits 188 -> 177 us.)  Elsewhere blocks ask line by
     // line for their own runs of k, in the order they will read them (rows as a whole instead:
     // output product 4.5 -> 7 us, a step with 8 192 x 2 048 products 1 % slower).
     pdl_trigger();
-    if (EPI == EPI_ROPE || ahead == 0 || K > 32768) {
+    if (EPI == EPI_ROPE || ahead == 0) {
         if (t == 0) {
             for (int kb = (rank * 8 + warp) * 64; kb < K; kb += ksplit * 8 * 64) {
 #pragma unroll
@@ -336,6 +336,22 @@ skinny_linear_dense_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloa
     skinny_linear_body<1, 1, OutT, EPI>(W, x, y, R, N, K, x_stride, y_stride, cap, ksplit, ahead, rope);
 }
 
+// How many blocks on a block asks L2 for the weight rows of the one that takes its place (0: not at all): `resident`
+// blocks of `tile` rows of K elements run at a time, on a device with `l2` bytes of L2.  What all of them ask
+// for has to stay in L2 beside what they read: 3/8 of it at most (126 MB: widths up to 2 560; at 2 688 the logits
+// of 256 000 rows take 245 us with it and 233 without, at 3 584 378 and 301).  It pays where one such request
+// covers the rest of the grid, one and a half to two times what is resident (in a chain of products, 8 rows,
+// without -> with: 16 384 x 2 048 17.2 -> 16.8 us, 18 432 x 2 304 20.8 -> 20.0), and where the grid is long and its rows are
+// too (256 000 x 2 304 194 -> 183, 128 000 x 2 304 102 -> 98, 256 000 x 2 048 165 -> 161).  Between the two it costs
+// more than it brings (24 576 x 2 304 26.3 -> 26.5, 32 000 x 2 048 26.8 -> 28.1, 65 536 x 2 048 48.0 -> 49.2), as
+// with short rows (256 000 x 1 536 118 -> 123) and a grid that hardly overflows (12 288 x 2 048 14.5 -> 15.0).
+SIB_EXPORT int sib_skinny_linear_ahead(int blocks, int resident, int tile, int K, int l2) {
+    if (resident <= 0 || blocks <= resident || 2ll * resident * tile * K > l2 / 8 * 3ll) return 0;
+    const bool rest = 2ll * blocks >= 3ll * resident && blocks <= 2 * resident;
+    const bool long_grid = blocks >= 12 * resident && K >= 2048;
+    return rest || long_grid ? resident : 0;
+}
+
 template <int NT, int MT, typename OutT, int EPI>
 static int launch_skinny(const void* W, const void* x, void* y, int R, int N, int K, int x_stride,
                          int y_stride, float cap, const RopeTail& rope, cudaStream_t s) {
@@ -382,14 +398,19 @@ static int launch_skinny(const void* W, const void* x, void* y, int R, int N, in
     }
     // More blocks than the device holds at a time: how many come before the one that takes a block's place.
     int ahead = 0;
-    if (ksplit == 1 && blocks > 2 * sms) {
-        static int per_sm = 0;       // (of this instantiation's two kernels the one that takes such grids)
-        if (!per_sm && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, skinny_linear_kernel<NT, MT, OutT, EPI>, 256,
-                                                                     smem) != cudaSuccess)
-            per_sm = 1;
-        // (what all blocks ask for ahead has to stay in L2 beside what they read: 44 MB at a width of 2 304; at
-        // 3 584 it would be 68 MB of 126, and the logits of that width took 80 us more with it)
-        if (blocks > per_sm * sms && (long long)per_sm * sms * 16 * MT * K * 2 <= (48ll << 20)) ahead = per_sm * sms;
+    if (ksplit == 1 && blocks > sms) {
+        // (of the first device asked, as above; of this instantiation's two kernels the one that takes such grids)
+        static const int per_sm = [&] {
+            int n = 0;
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, skinny_linear_kernel<NT, MT, OutT, EPI>, 256, smem) ==
+                           cudaSuccess ? n : 0;
+        }();
+        static const int l2 = [&] {
+            int dev = 0, n = 0;
+            return cudaGetDevice(&dev) == cudaSuccess &&
+                           cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) == cudaSuccess ? n : 0;
+        }();
+        ahead = sib_skinny_linear_ahead(blocks, per_sm * sms, 16 * MT, K, l2);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks, ksplit, 1);

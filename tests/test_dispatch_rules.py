@@ -40,3 +40,14 @@ def test_a_scan_goes_row_by_row_where_the_memory_of_its_chunks_cannot_be_had(mon
     assert native.chunked_scan_scratch(out, ctx, 8, 128, 256) is not None
     monkeypatch.setattr(native.torch, "empty", empty)
     assert native.chunked_scan_scratch(out, ctx, 8, 128, 256) is None
+
+
+def test_few_row_products_ask_ahead_where_that_pays():
+    def ahead(N, K, resident=592, l2=126 << 20):
+        return native.library().sib_skinny_linear_ahead(*map(c_int, (-(-N // 16), resident, 16, K, l2)))
+
+    assert ahead(18432, 2304) == ahead(16384, 2048) == ahead(256000, 2304) == ahead(128000, 2048) == 592
+    for N, K in ((9216, 2304), (12288, 2048), (24576, 2304), (32000, 2048), (65536, 2048), (256000, 1536),
+                 (256000, 2688), (18432, 3584), (256000, 1 << 20)):
+        assert ahead(N, K) == 0, (N, K)
+    assert ahead(256000, 2304, l2=96 << 20) == 0 and ahead(256000, 2304, resident=0) == 0
