@@ -1002,8 +1002,8 @@ def test_sampling_with_ties_at_the_edge_of_top_k(n_top, top_k, top_p):
 @pytest.mark.parametrize("place", ["spread", "one thread", "one block", "few finite"])
 def test_sampling_of_the_top_k_wherever_they_lie(vocab, top_k, top_p, place):
     """The threads' maxima bound the k-th largest logit well where the largest are spread over the threads
-    and badly where one thread holds them all (then everything above the bound does not fit the
-    list); with fewer finite logits than top-k there is no bound."""
+    and less well where one thread or block holds them all (at these sizes a thread has 8 elements at most, so what lies
+    above the bound still fits the list); with fewer finite logits than top-k there is no bound."""
     n = _native()
     g = torch.Generator().manual_seed(31)
     logits = torch.randn(vocab, generator=g)
@@ -1021,6 +1021,29 @@ def test_sampling_of_the_top_k_wherever_they_lie(vocab, top_k, top_p, place):
     state = torch.tensor([77], dtype=torch.int64, device=DEV)
     out = torch.empty(1, dtype=torch.int32, device=DEV)
     rng, differ = plain.XorShift64(77), 0
+    for _ in range(20):
+        n.sample_rows(dev, 0.9, top_k, top_p, state, out)
+        differ += plain.sample_token(logits, 0.9, top_k, top_p, rng) != int(out)
+    assert differ <= 1, f"{differ} of 20 draws differ from the plain sampler"
+
+
+@pytest.mark.parametrize("top_p", [1.0, 0.9])
+def test_sampling_where_too_many_lie_above_the_bound(top_p):
+    """The 20 threads that hold the largest logits hold over a thousand of them, and top-k asks for more maxima than 20:
+    what lies above the bound does not fit the list, and the row is searched."""
+    n = _native()
+    g = torch.Generator().manual_seed(37)
+    vocab, top_k, per_block = 256000, 40, 32000
+    # (the rest in a narrow band far below: the bound is one of its threads' maxima)
+    logits = -6.0 + 0.01 * torch.rand(vocab, generator=g)
+    held = torch.cat([torch.arange(per_block * 2 + 9 * t, per_block * 3, 512) for t in range(20)])
+    logits[held] = 5.0 + 2.0 * torch.randn(held.numel(), generator=g)
+    maxima = torch.stack([logits[per_block * b + t:per_block * (b + 1):512].max() for b in range(8) for t in range(512)])
+    assert int((logits >= maxima.topk(top_k).values[-1]).sum()) > 256
+    dev = logits[None].to(DEV)
+    state = torch.tensor([91], dtype=torch.int64, device=DEV)
+    out = torch.empty(1, dtype=torch.int32, device=DEV)
+    rng, differ = plain.XorShift64(91), 0
     for _ in range(20):
         n.sample_rows(dev, 0.9, top_k, top_p, state, out)
         differ += plain.sample_token(logits, 0.9, top_k, top_p, rng) != int(out)
