@@ -243,14 +243,20 @@ __global__ void __launch_bounds__(128) delta_prepare_runs_kernel(DeltaPrepareArg
 // The history after the step: the last taps - 1 inputs of each sequence.  One thread per
 // (sequence, channel) walks the cells oldest first; a cell that keeps an older input takes
 // it from a later cell of the same history, which has not been rewritten yet.
+// `late`: the kernel behind this one may begin once the one ahead has finished, not at once.  A scan over
+// prompts is a few hundred warps that wait for latencies all the time; begun under the last blocks of
+// what makes its inputs, several of its blocks share the SMs that happen to be free and stay there (inputs, scan and
+// norm of the delta rule, early -> late: 2 048 rows of 8 heads of 128 x 256 1 345 -> 720 us, of 16 heads of 128 x 128
+// 1 389 -> 770, 128 rows 111 -> 72, 16 rows 40 -> 37).
 template <typename T>
 __global__ void conv_history_kernel(const T* __restrict__ proj, long long stride, float* state,
                                     long long state_stride, long long hist_offset,
                                     const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                                     const int* __restrict__ seq_end, const int* __restrict__ seq_row0,
-                                    int channels, int taps) {
-    pdl_trigger();
+                                    int channels, int taps, bool late) {
+    if (!late) pdl_trigger();
     pdl_wait();
+    if (late) pdl_trigger();
     const int b = blockIdx.y;
     const int slot = seq_slot[b];
     if (slot < 0) return;
@@ -620,7 +626,8 @@ SIB_EXPORT int sib_delta_prepare(
                        row_seq, seq_slot, seq_start, seq_row0, stride, state_stride, hist_offset,
                        H, G, kd, vd, taps};
     cudaStream_t s = (cudaStream_t)stream;
-    if (sib_delta_prepare_in_runs(rows, n_seqs, H, G, kd, taps) && ((uintptr_t)conv_w % 16) == 0)
+    const bool in_runs = sib_delta_prepare_in_runs(rows, n_seqs, H, G, kd, taps) && ((uintptr_t)conv_w % 16) == 0;
+    if (in_runs)
         SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(delta_prepare_runs_kernel<T>,
                                                      dim3((rows + kRunRows - 1) / kRunRows, (units + 3) / 4), dim3(128), 0,
                                                      s, p, rows));
@@ -633,7 +640,7 @@ SIB_EXPORT int sib_delta_prepare(
     SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(conv_history_kernel<T>, grid, dim3(256), 0, s,
                                                  (const T*)proj, stride, state, state_stride,
                                                  hist_offset, seq_slot, seq_start, seq_end, seq_row0,
-                                                 channels, taps));
+                                                 channels, taps, rows >= 4ll * n_seqs));
     return sib_check_launch("conv_history");
 }
 
@@ -867,7 +874,7 @@ SIB_EXPORT int sib_ssm_prepare(const void* proj, long long stride, int dtype, co
     SIB_DISPATCH_DTYPE(dtype, sib_launch_chained(conv_history_kernel<T>, grid, dim3(256), 0, s,
                                                  (const T*)first, stride, state, state_stride,
                                                  hist_offset, seq_slot, seq_start, seq_end, seq_row0,
-                                                 channels, taps));
+                                                 channels, taps, false));
     return sib_check_launch("conv_history");
 }
 
