@@ -447,9 +447,12 @@ __device__ int sample_from_short_list(Cluster& c, const float* row, int lo, int 
     return token;
 }
 
-// (two blocks an SM: with one, which is what the registers of a build without a bound leave, 64 rows of the
-// cluster of 8 are four waves)
-__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, 2)
+// PER_SM: blocks an SM that the registers are to leave room for.  Two where not all rows' clusters of 8 have SMs to
+// themselves (with one, 16 rows are two waves and 64 are four: of 256 000, temperature alone, one -> two: 24 rows 43 -> 33
+// us, 64 rows 99 -> 67); one, and no register spilled, where they have, as two blocks were put on one SM all the
+// same (8 rows of 256 000, two -> one: temperature alone 26.3 -> 23.4 us, top-p alone 176 -> 156).
+template <int PER_SM>
+__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, PER_SM)
 sample_rows_kernel(SampleArgs p) {
     extern __shared__ __align__(16) unsigned char sample_smem[];
     SampleShared* sh = reinterpret_cast<SampleShared*>(sample_smem);
@@ -678,14 +681,25 @@ SIB_EXPORT int sib_sample_rows(const float* logits, long long stride, int rows, 
     SIB_REQUIRE(top_k >= 0 && top_p > 0.f, "sample_rows: top_k=%d top_p=%f", top_k, top_p);
     SampleArgs p{logits, stride, vocab, temperature, top_k, top_p, rng, rng_index, out};
     const size_t smem = sizeof(SampleShared);
-    cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // how many rows' clusters run at a time with an SM for every block (of the first device asked: a matter of speed)
+    static const int alone = [smem] {
+        int n = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(SAMPLE_CLUSTER, 1);
+        cfg.blockDim = dim3(SAMPLE_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        const bool ok = cudaFuncSetAttribute(sample_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+                            cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, sample_rows_kernel<1>, &cfg) == cudaSuccess;
+        return ok ? n : 0;
+    }();
+    auto kernel = rows <= alone ? sample_rows_kernel<1> : sample_rows_kernel<2>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
         sib_set_error("sample_rows: shared memory: %s", cudaGetErrorString(e));
         return (int)e;
     }
-    e = sib_launch_chained(sample_rows_kernel, dim3(SAMPLE_CLUSTER, rows), dim3(SAMPLE_THREADS),
-                           smem, (cudaStream_t)stream, p);
+    e = sib_launch_chained(kernel, dim3(SAMPLE_CLUSTER, rows), dim3(SAMPLE_THREADS), smem, (cudaStream_t)stream, p);
     if (e != cudaSuccess) {
         sib_set_error("sample_rows: launch failed: %s", cudaGetErrorString(e));
         return (int)e;
