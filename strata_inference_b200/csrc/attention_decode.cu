@@ -164,7 +164,7 @@ constexpr int MAX_SHARED_ROWS = 128;
 
 // A step's sequences are seldom equally long, and a launch that cuts every row into the same
 // number of runs lasts as long as the longest row's: 64 sequences of 150 to 3 001 positions (4 kv
-// heads of 256) took 98 us where their keys and values take 38 at the copy bandwidth.  So every
+// heads of 256) took 90 us where their keys and values take 38 at the copy bandwidth (shared out: 57).  So every
 // block finds its place itself: with `each` tiles a warp, row r gets ceil(tiles_r / (nw each))
 // blocks per kv head, and `each` is the smallest number at which that fits the `slots` blocks
 // there are (all resident at once) and no row needs more than MAX_SPLITS.  It depends on the rows'
@@ -232,8 +232,11 @@ __device__ __forceinline__ bool share_out(const AttnDecodeArgs& p, int slot, int
 // blocks of 4); the narrower kernel keeps its registers and shared memory as they were.
 // SHARED: the blocks of a kv head are shared out by the rows' lengths (share_out), else every row
 // has `splits` of them.
+// (SHARED with 4 heads of 256 a group: bound to the registers of the even kernel, of whose blocks an SM holds three; left
+// to itself the compiler takes 235, an SM holds two, and the blocks that should all be resident are two waves)
 template <int HD, int G, bool EARLY, bool WIDE = false, bool SHARED = false>
-__global__ void __launch_bounds__(WIDE ? 256 : 128) attention_decode_kernel(AttnDecodeArgs p) {
+__global__ void __launch_bounds__(WIDE ? 256 : 128, SHARED && HD == 256 && G == 4 ? 3 : 0)
+attention_decode_kernel(AttnDecodeArgs p) {
     constexpr int KB = HD / 32;          // 32-wide blocks of the head dimension
     constexpr int LPK = HD / 8;          // lanes that cover one value row
     constexpr int KPP = 32 / LPK;        // keys per pass of the weighted sum
@@ -546,7 +549,7 @@ SIB_EXPORT int sib_attention_decode_supports(int n_heads, int n_kv, int head_dim
 // How many warps of this kernel the current device holds at a time for the shape (blocks of
 // 4 warps that fit on an SM, by the kernel's registers and shared memory, times the SMs):
 // what a caller sizes its split of the keys by.  0 if the shape is not one this kernel takes.
-static int resident_warps(int n_heads, int n_kv, int head_dim, int warps);
+static int resident_warps(int n_heads, int n_kv, int head_dim, int warps, bool shared = false);
 
 SIB_EXPORT int sib_attention_decode_resident_warps(int n_heads, int n_kv, int head_dim) {
     return resident_warps(n_heads, n_kv, head_dim, 4);
@@ -558,7 +561,12 @@ SIB_EXPORT int sib_attention_decode_resident_warps_of(int n_heads, int n_kv, int
     return resident_warps(n_heads, n_kv, head_dim, warps);
 }
 
-static int resident_warps(int n_heads, int n_kv, int head_dim, int warps) {
+// ... and for blocks of 4 warps that are shared out by the rows' lengths.
+SIB_EXPORT int sib_attention_decode_shared_resident_warps(int n_heads, int n_kv, int head_dim) {
+    return resident_warps(n_heads, n_kv, head_dim, 4, true);
+}
+
+static int resident_warps(int n_heads, int n_kv, int head_dim, int warps, bool shared) {
     if (!sib_attention_decode_supports(n_heads, n_kv, head_dim, 16)) return 0;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -577,7 +585,8 @@ static int resident_warps(int n_heads, int n_kv, int head_dim, int warps) {
                   &per_sm, attention_decode_kernel<HD, GG, false, true>, 256,               \
                   (size_t)8 * GG * (HD + 2) * sizeof(float))                                \
             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(                                \
-                  &per_sm, attention_decode_kernel<HD, GG, false>, 32 * warps,              \
+                  &per_sm, shared ? attention_decode_kernel<HD, GG, false, false, true>     \
+                                  : attention_decode_kernel<HD, GG, false>, 32 * warps,     \
                   (size_t)warps * GG * (HD + 2) * sizeof(float))
 #define BY_G(HD)                    \
     do {                            \

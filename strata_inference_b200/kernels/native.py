@@ -1645,6 +1645,11 @@ def attention_decode_resident_warps(n_heads: int, n_kv: int, head_dim: int, warp
                                                                 c_int(head_dim), c_int(warps)))
 
 
+def attention_decode_shared_resident_warps(n_heads: int, n_kv: int, head_dim: int) -> int:
+    """The same of the kernel whose blocks are shared out by the rows' lengths, in blocks of 4 warps."""
+    return int(library().sib_attention_decode_shared_resident_warps(c_int(n_heads), c_int(n_kv), c_int(head_dim)))
+
+
 # 32-bit prompts whose longest has at least this many rows go to the tiled kernel (16 prompts, 8 heads of 256,
 # tiled against the general kernel: of 2 rows 16 and 10 us, of 5 rows 16 and 12, of 16 rows 18 and 21, of 32
 # rows 18 and 43)

@@ -436,7 +436,7 @@ class Attention:
         tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
         shares = not rt.steady_sums and (self.window == 0 or self.window >= 2048)
         if shares and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
-            shared = shared_shape(R, self.nkv, tiles, self._resident_warps[4])
+            shared = shared_shape(R, self.nkv, tiles, self._resident_warps["shared"])
             if shared is not None:
                 slots, warps = shared
                 scratch = rt.scratch(native.attention_rows_scratch_bytes(1, self.nh, self.kw, slots))
@@ -464,6 +464,7 @@ class Attention:
         if self._resident_warps is None:     # what the device holds of this kernel at a time
             self._resident_warps = {w: native.attention_decode_resident_warps(self.nh, self.nkv, self.kw, w)
                                     for w in (8, 4)}
+            self._resident_warps["shared"] = native.attention_decode_shared_resident_warps(self.nh, self.nkv, self.kw)
         # (a chunk that does not begin at a tile's first key reaches into one tile more, as a window does)
         edge = (self.window + -(-self.keep // 16) * 16 if self.window else 0) or (self.chunk if self.chunk % 16 else 0)
         return decode_shape(max(1, ctx.n_rows * self.nkv), self._longest(ctx, capacity), edge,

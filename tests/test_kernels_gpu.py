@@ -279,6 +279,14 @@ def test_attention_decode_shared_out(nh, nkv, hd, window, cap, slots, warps, pic
         _close(out[i].view(nh, hd), want, dtype, f"row {r}")
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+def test_attention_decode_shared_out_fits_the_device_as_even_runs_do(hd, group):
+    """Blocks that are shared out should all be resident at once: an SM holds as many of them as of the even kernel's."""
+    n = _native()
+    assert n.attention_decode_shared_resident_warps(group, 1, hd) >= n.attention_decode_resident_warps(group, 1, hd)
+
+
 @pytest.mark.parametrize("nh,nkv,hd,window,cap", [
     (4, 2, 64, 0, 0.0), (8, 4, 256, 100, 50.0), (4, 1, 128, 0, 30.0), (2, 2, 128, 70, 0.0),
     (8, 4, 256, 0, 0.0), (3, 3, 64, 17, 20.0)])
