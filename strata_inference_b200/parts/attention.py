@@ -156,19 +156,19 @@ def decode_shape(units: int, longest: int, window: int, resident4: int, resident
     return trimmed(min(most, 128), 1)
 
 
-def shared_shape(rows: int, n_kv: int, tiles: int, resident: int):
+def shared_shape(rows: int, n_kv: int, tiles: int, resident: int, least: int = 1):
     """(blocks per kv head, warps a block) of the decode kernel for ``rows`` rows of up to ``tiles``
     tiles of 16 keys that share the blocks out by their lengths, on a device that holds
-    ``resident`` warps of the kernel; None where not even blocks of one warp go round.  Wide blocks
+    ``resident`` warps of the kernel; None where not even blocks of ``least`` warps go round.  Wide blocks
     leave fewer partial results to join, narrow ones divide the keys more evenly: a narrower one is
     taken where a warp of equally long rows would walk a fifth fewer tiles (64 rows of 3 000
     positions, 4 kv heads of 256: 128 us with 2 warps, 140 with 4; 16 rows of 1 000: 21 with 2, 17 with
     4), or where the wider blocks are hardly more than the rows and lengths could not count (100
     rows of 64 to 7 000 positions, 8 kv heads of 256: 188 us with 1 warp, 297 with 2)."""
     best, best_each = None, 0
-    for warps in (4, 2, 1):
+    for warps in (w for w in (4, 2, 1) if w >= least):
         slots = resident // (warps * n_kv)
-        if slots < rows or (warps > 1 and slots < 1.5 * rows):
+        if slots < rows or (warps > least and slots < 1.5 * rows):
             continue
         each = -(-tiles // (slots // rows * warps))
         if best is None or each <= 0.8 * best_each:
@@ -433,10 +433,14 @@ class Attention:
         # A model with parts that make much of a last bit keeps even runs (Runtime.steady_sums): shared out, the order
         # of a row's sums would depend on the other rows' lengths (decode steps of a Karupel of 8 layers: logits
         # up to 3 % apart; what that costs: 32 rows of 150 to 3 001 positions, 16 heads on 8 kv heads of 128, 64 us instead of 35).
+        # Rows that turn out equally long pay for the joins: up to 512 positions 0 to 6 % with blocks as wide as the even
+        # runs' and up to 22 % with narrower ones, which short steps therefore do not take (8 heads on 4 kv heads of 256,
+        # 96 rows of 500 positions: 38 us even, 46 in blocks of 2 warps); of 4 000 positions 3 % on average, 11 % at
+        # most, level where the mean is 0.9 of the longest, 13 % faster (up to 35 %) where it is 0.65.
         tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
         shares = not rt.steady_sums and (self.window == 0 or self.window >= 2048)
         if shares and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
-            shared = shared_shape(R, self.nkv, tiles, self._resident_warps["shared"])
+            shared = shared_shape(R, self.nkv, tiles, self._resident_warps["shared"], warps if tiles < 128 else 1)
             if shared is not None:
                 slots, warps = shared
                 scratch = rt.scratch(native.attention_rows_scratch_bytes(1, self.nh, self.kw, slots))

@@ -63,3 +63,10 @@ def test_shared_blocks_are_wide_where_that_costs_no_tiles():
     assert shared_shape(64, 4, 7, RES4) == (111, 4)         # short rows: one block each
     assert shared_shape(64, 4, 188, RES4) == (222, 2)
     assert shared_shape(100, 8, 257, RES4) == (222, 1)      # blocks of 2: hardly more than rows
+
+
+def test_shared_blocks_of_short_steps_are_no_narrower_than_even_runs():
+    assert shared_shape(96, 4, 32, RES4) == (222, 2)
+    assert shared_shape(96, 4, 32, RES4, least=4) == (111, 4)       # one block each for equal rows, as even runs
+    assert shared_shape(64, 4, 32, RES4, least=2) == (222, 2)
+    assert shared_shape(128, 4, 32, RES4, least=4) is None
