@@ -19,14 +19,12 @@
 //                 chunk_pass      S' = A_C S + B, element by element; keeps every S
 //   all           chunk_out       P[t, s] = D(t, s) (q_t . k_s);  O = P U + A Q S
 //
-// Measured (one sequence, 8 heads of 128 x 256, token by token -> in chunks): 2 048
-// tokens, delta rule 632 -> 268 us, memory 768 -> 230, gated 574 -> 172; 512 tokens, delta rule 171 -> 104; 128 tokens
-// 56 -> 83, hence the least number of rows in kernels/native.py; eight sequences of 2 048, delta rule 2 267 -> 1 539.
-// (With the products that make the outputs inside the walk, and the matrix in registers as 2 x 4 a thread:
-// 285, 253, 237, 112, 76 and 1 798 us.)
-// All of it is bound by shared memory's bandwidth: a thread's tile of 8 x 4 loads a word for 2.7
-// FMAs.  Against 64 bits the outputs are 1.6e-7 off (token by token 0.9e-7), the matrices
-// 5.5e-8 (5.4e-8).
+// Measured (8 heads of 128 x 256, token by token -> in chunks): one sequence of 2 048 tokens, delta rule 702 -> 255 us,
+// gated 639 -> 163; of 300 tokens 111 -> 93 and 101 -> 60; of 160 tokens 63 -> 87 and 58 -> 56; eight of 300 341 ->
+// 325 and 309 -> 214 (more in kernels/native.py, beside the rule). All of it is bound by shared memory's bandwidth: a
+// thread's tile of 8 x 4 loads a word for 2.7 FMAs.  Against 64 bits the outputs are 1.3e-7 to 1.7e-7 off (token by
+// token 0.9e-7), the matrices 7e-8 (6e-8).  That is further than before, so the engine's parts take these kernels
+// only where an engine's owner asks for them (parts/base.py Runtime.chunked_scans).
 //
 // The decays enter as products of the given factors, never as differences of logarithms or quotients:
 // a factor of 0 is an ordinary value.  All sums are 32-bit FMAs; pairs of them issue as one
@@ -38,7 +36,7 @@
 namespace {
 
 constexpr int C = 64;            // tokens of a chunk
-constexpr int NT = 256;          // threads of a block, in both kernels
+constexpr int NT = 256;          // threads of a block of chunk_prepare and chunk_walk
 constexpr int MS = C + 4;        // row stride of a C x C matrix in shared memory
 constexpr int CB = 16;           // columns of a block of the walk
 

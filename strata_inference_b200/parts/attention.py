@@ -433,10 +433,11 @@ class Attention:
         # A model with parts that make much of a last bit keeps even runs (Runtime.steady_sums): shared out, the order
         # of a row's sums would depend on the other rows' lengths (decode steps of a Karupel of 8 layers: logits
         # up to 3 % apart; what that costs: 32 rows of 150 to 3 001 positions, 16 heads on 8 kv heads of 128, 64 us instead of 35).
-        # Rows that turn out equally long pay for the joins: up to 512 positions 0 to 6 % with blocks as wide as the even
-        # runs' and up to 22 % with narrower ones, which short steps therefore do not take (8 heads on 4 kv heads of 256,
-        # 96 rows of 500 positions: 38 us even, 46 in blocks of 2 warps); of 4 000 positions 3 % on average, 11 % at
-        # most, level where the mean is 0.9 of the longest, 13 % faster (up to 35 %) where it is 0.65.
+        # Rows that turn out equally long pay for the joins: of 500 positions 0 to 6 % with blocks as wide as the even
+        # runs' and up to 22 % with narrower ones, which steps of fewer than 2 048 positions therefore do not take (8
+        # heads on 4 kv heads of 256, 96 rows, even -> blocks of 2 warps: of 500 positions 38 -> 46 us, of 1 000 66 -> 74);
+        # of 4 000 positions 3 % on average, 11 % at most, level where the mean is 0.9 of the longest, 13 % faster (up to
+        # 35 %) where it is 0.65.
         tiles = -(-self._longest(ctx, ctx.cache.max_seq_len) // 16)
         shares = not rt.steady_sums and (self.window == 0 or self.window >= 2048)
         if shares and warps < 8 and tiles > 2 * runs * warps and 1 < R <= native.attention_decode_max_shared_rows():
